@@ -35,9 +35,6 @@
 #ifndef DGR_MINB_EDGE
 #define DGR_MINB_EDGE (768 / DGR_EDGE_BS)
 #endif
-/* 1: the edge and limiter kernels take their divisions through shared reciprocals
- * (div_rcp), queueing the items where that is not valid for a plain-division redo launch;
- * 0: plain divisions.  Chosen by measurement, overridable at build time. */
 /* Resident threads per SM requested for the limiter kernel (register cap 65536 / this);
  * chosen by measurement (1024: 64 registers, 0.244 ms at 4M triangles; 768: 80 registers,
  * 0.271 ms; 512: 0.350 ms). */
@@ -48,12 +45,6 @@
  * 128 registers at 512). */
 #ifndef DGR_ELEMENT_THREADS_PER_SM
 #define DGR_ELEMENT_THREADS_PER_SM 512
-#endif
-#ifndef DGR_EDGE_RCP
-#define DGR_EDGE_RCP 1
-#endif
-#ifndef DGR_LIMIT_RCP
-#define DGR_LIMIT_RCP 1
 #endif
 
 namespace dgr {
@@ -104,7 +95,6 @@ struct MeshDev {
     const int *ed_sid;    /* scenario of each edge, NULL for a single mesh */
     int flux;             /* numerical flux: 0 Roe (2DCode), 1 local Lax-Friedrichs, 2 HLLC (DG-SWEM) */
     unsigned long long *bad_index; /* checked build: first out-of-range gather, (kernel << 32 | item) */
-    int *redo;            /* edges left to k_edge_redo: [0] count, [1] blocks done, [2..] edges */
 };
 
 /* Checked build (compiled with -DDGR_CHECKED): every index a kernel gathers from the
@@ -167,14 +157,27 @@ DGR_DEV void prefetch_geometry(const MeshDev &m, int base, int n)
 /* One edge (2DCode/compute2DL.c:17-331): traces, ghost state, Roe flux(es); stores Fhat.n
  * for both sides and returns the edge's max wave speed (0 for a finished scenario).
  * FT: the numerical flux as a compile-time constant (0 Roe, 1 LLF, 2 HLLC), or -1 to take
- * it from the mesh at run time.  With `redo` non-null the Roe flux's divisions share one
- * reciprocal per divisor (RcpDiv, the same bits); an edge where that is not valid reports
- * no error and no speed and sets *redo: the caller queues it for k_edge_redo, which
- * redoes it with plain divisions in a launch of its own and overwrites its fluxes. */
-template <bool WD, bool COH = false, int FT = -1>
+ * it from the mesh at run time.  RCP: the Roe flux's divisions share one reciprocal per
+ * divisor (RcpDiv, the same bits); an edge where that is not valid is redone by
+ * edge_item_plain (plain divisions, kept out of line). */
+template <bool WD, bool COH = false, int FT = -1, bool RCP = false>
 DGR_DEV double edge_flux_item(const MeshDev &m, const double *S, const int *wd, const double *bzeta,
-                              const double *bqn, double *flux, DevClock *clk, int phase, double g, int i,
-                              bool *redo = nullptr)
+                              const double *bqn, double *flux, DevClock *clk, int phase, double g, int i);
+
+/* Inside the same launch: a queue and a redo launch of their own after every edge and limiter
+ * kernel cost 3.5 us each with nothing queued (a step of 1,600 triangles 3.88 -> 3.36 ms per
+ * 60 steps without them, 200k 25.0 -> 23.6 ms per 100, 4M 2.34 -> 2.31 ms per step). */
+template <bool WD, int FT>
+__device__ __noinline__ double edge_item_plain(const MeshDev &m, const double *S, const int *wd, const double *bzeta,
+                                               const double *bqn, double *flux, DevClock *clk, int phase, double g,
+                                               int i)
+{
+    return edge_flux_item<WD, false, FT>(m, S, wd, bzeta, bqn, flux, clk, phase, g, i);
+}
+
+template <bool WD, bool COH, int FT, bool RCP>
+DGR_DEV double edge_flux_item(const MeshDev &m, const double *S, const int *wd, const double *bzeta,
+                              const double *bqn, double *flux, DevClock *clk, int phase, double g, int i)
 {
     double lam = 0.0;
     DevClock *ck = clk + (m.ed_sid ? m.ed_sid[i] : 0);
@@ -201,15 +204,11 @@ DGR_DEV double edge_flux_item(const MeshDev &m, const double *S, const int *wd, 
         const int wdi = WD ? ldm<COH>(&wd[el_in]) : 1, wde = WD ? ldm<COH>(&wd[el_ex]) : 1;
         double fin[3], fex[3];
         int code;
-        if (redo) {
+        if constexpr (RCP) {
             RcpDiv dv;
             lam = flux_core<double, WD, RcpDiv>(zi, qxi, qyi, ze, qxe, qye, z_edge, nx, ny, wdi, wde, g, fin, fex,
                                                 code, FT >= 0 ? FT : m.flux, &dv);
-            if (!dv.ok) { /* k_edge_redo rewrites this edge's fluxes, error and speed */
-                *redo = true;
-                code = 0;
-                lam = 0.0;
-            }
+            if (!dv.ok) return edge_item_plain<WD, FT>(m, S, wd, bzeta, bqn, flux, clk, phase, g, i);
         } else {
             lam = flux_core<double, WD>(zi, qxi, qyi, ze, qxe, qye, z_edge, nx, ny, wdi, wde, g, fin, fex, code,
                                         FT >= 0 ? FT : m.flux);
@@ -266,40 +265,9 @@ __global__ void __launch_bounds__(DGR_EDGE_BS, DGR_MINB_EDGE) k_edge_flux(const 
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = i < m.nf;
     const int sid = (valid && m.ed_sid) ? m.ed_sid[i] : 0;
-    bool redo = false;
     const double lam =
-        valid ? edge_flux_item<WD, false, FT>(m, S, wd, bzeta, bqn, flux, clk, phase, g, i,
-                                              DGR_EDGE_RCP ? &redo : nullptr)
-              : 0.0;
-    if (redo) m.redo[2 + atomicAdd(&m.redo[0], 1)] = i;
+        valid ? edge_flux_item<WD, false, FT, FT == 0>(m, S, wd, bzeta, bqn, flux, clk, phase, g, i) : 0.0;
     block_max_speed(lam, sid, valid, clk, lam_slot);
-}
-
-/* The edges k_edge_flux queued (m.redo: [0] count, [1] blocks done, [2..] edges), with
- * plain divisions: fluxes, error and wave speed as k_edge_flux would have given them.
- * Launched after every k_edge_flux; with nothing queued each block returns at once.  The
- * last block to finish clears the queue for the next launch. */
-template <bool WD, int FT>
-__global__ void __launch_bounds__(256) k_edge_redo(const __grid_constant__ MeshDev m, const double *__restrict__ S,
-                                                   const int *__restrict__ wd, const double *__restrict__ bzeta,
-                                                   const double *__restrict__ bqn, double *__restrict__ flux,
-                                                   DevClock *clk, int lam_slot, int phase, double g)
-{
-    const int n = *(volatile int *)&m.redo[0];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const int i = m.redo[2 + k];
-        const double lam = edge_flux_item<WD, false, FT>(m, S, wd, bzeta, bqn, flux, clk, phase, g, i);
-        const int sid = m.ed_sid ? m.ed_sid[i] : 0;
-        if (lam > 0.0) atomicMax(&clk[sid].lam_bits[lam_slot], (unsigned long long)__double_as_longlong(lam));
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(&m.redo[1], 1) == (int)gridDim.x - 1) {
-            m.redo[0] = 0;
-            m.redo[1] = 0;
-        }
-    }
 }
 
 /* ---------------------------------------------------------------- elements ---- */
@@ -469,6 +437,20 @@ static __global__ void __launch_bounds__(256) k_wd_status(MeshDev m, const doubl
  */
 template <bool LIMIT, bool PDOP, bool STATUS, bool COH = false, bool RCP = false>
 DGR_DEV void limit_item(const MeshDev &m, double *S, const double *bounds, const int *wd_in, int *wd_out,
+                        DevClock *clk, double h0, double velzero, int phase, int *dec_limit, int *dec_pdop, int el);
+
+/* an element where the shared reciprocals are not valid, with plain divisions, kept out of
+ * line: its state is still untouched */
+template <bool LIMIT, bool PDOP, bool STATUS>
+__device__ __noinline__ void limit_item_plain(const MeshDev &m, double *S, const double *bounds, const int *wd_in,
+                                              int *wd_out, DevClock *clk, double h0, double velzero, int phase,
+                                              int *dec_limit, int *dec_pdop, int el)
+{
+    limit_item<LIMIT, PDOP, STATUS>(m, S, bounds, wd_in, wd_out, clk, h0, velzero, phase, dec_limit, dec_pdop, el);
+}
+
+template <bool LIMIT, bool PDOP, bool STATUS, bool COH, bool RCP>
+DGR_DEV void limit_item(const MeshDev &m, double *S, const double *bounds, const int *wd_in, int *wd_out,
                         DevClock *clk, double h0, double velzero, int phase, int *dec_limit, int *dec_pdop, int el)
 {
     DevClock *ck = clk + (m.el_sid ? m.el_sid[el] : 0);
@@ -492,8 +474,9 @@ DGR_DEV void limit_item(const MeshDev &m, double *S, const double *bounds, const
     RcpDiv dv;
     if constexpr (RCP) {
         limit_core<LIMIT, PDOP, double, decltype(bnd), false, RcpDiv>(w, bnd, zn, h0, velzero, dec, nullptr, &dv);
-        if (!dv.ok) { /* k_limit_redo redoes it with plain divisions from the untouched state */
-            m.redo[2 + atomicAdd(&m.redo[0], 1)] = el;
+        if (!dv.ok) {
+            limit_item_plain<LIMIT, PDOP, STATUS>(m, S, bounds, wd_in, wd_out, clk, h0, velzero, phase, dec_limit,
+                                                  dec_pdop, el);
             return;
         }
     } else {
@@ -529,31 +512,8 @@ __global__ void __launch_bounds__(BS, DGR_LIMIT_THREADS_PER_SM / BS) k_limit(con
 {
     const int el = blockIdx.x * BS + threadIdx.x;
     if (el < m.ne)
-        limit_item<LIMIT, PDOP, STATUS, false, DGR_LIMIT_RCP>(m, S, bounds, wd_in, wd_out, clk, h0, velzero, phase,
-                                                             dec_limit, dec_pdop, el);
-}
-
-/* The elements k_limit queued (m.redo, as k_edge_redo), with plain divisions, from their
- * state as k_limit left it (untouched).  The last block to finish clears the queue. */
-template <bool LIMIT, bool PDOP, bool STATUS>
-__global__ void __launch_bounds__(128) k_limit_redo(const __grid_constant__ MeshDev m, double *__restrict__ S,
-                                                    const double *__restrict__ bounds, const int *__restrict__ wd_in,
-                                                    int *__restrict__ wd_out, DevClock *clk, double h0,
-                                                    double velzero, int phase, int *__restrict__ dec_limit,
-                                                    int *__restrict__ dec_pdop)
-{
-    const int n = *(volatile int *)&m.redo[0];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
-        limit_item<LIMIT, PDOP, STATUS>(m, S, bounds, wd_in, wd_out, clk, h0, velzero, phase, dec_limit, dec_pdop,
-                                        m.redo[2 + k]);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(&m.redo[1], 1) == (int)gridDim.x - 1) {
-            m.redo[0] = 0;
-            m.redo[1] = 0;
-        }
-    }
+        limit_item<LIMIT, PDOP, STATUS, false, true>(m, S, bounds, wd_in, wd_out, clk, h0, velzero, phase, dec_limit,
+                                                     dec_pdop, el);
 }
 
 /* ------------------------------------------------------------------ clock ---- */
