@@ -9,6 +9,7 @@
 
 #include <cstdio>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -91,7 +92,7 @@ struct dgr_ctx {
     /* schedule of the device loop */
     int bs;     /* block size of element/limiter work: 64, 128 or 256 */
     int fusion; /* 0, 1 or 2 */
-    cudaGraph_t graph;
+    cudaGraph_t graph; /* kGraphSteps steps of the device loop */
     cudaGraphExec_t graph_exec;
     cudaGraph_t stage_graph;          /* the RK stages of one dgr_step, without the clock */
     cudaGraphExec_t stage_graph_exec;
@@ -184,6 +185,24 @@ static inline StageIO stage_io(const dgr_ctx *c, int stage)
 /* flags the reference's WD array holds after a step: the last stage's input */
 static inline int *wd_after_step(const dgr_ctx *c) { return c->p.rk_stages == 3 ? c->wdC : c->wdB; }
 
+
+/* kernel launch that may start while the kernel before it in the stream finishes
+ * (programmatic stream serialization): for kernels that call pdl_wait before they read or
+ * write anything an earlier kernel writes.  A failure shows in cudaGetLastError, as with <<<>>>. */
+template <class... P, class... A>
+static inline void launch_dep(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t s, A &&...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 /* dgr_capi.cu */
 void drop_graph(dgr_ctx *c);

@@ -59,6 +59,17 @@ DGR_DEV T ldm(const T *p)
     return *p;
 }
 
+/* Dependent launch: the step's kernels are launched with programmatic stream serialization
+ * (launch_dep in dgr_internal.cuh), so a kernel's blocks may start while the kernel before it
+ * finishes.  pdl_wait returns once every earlier kernel of the stream has completed and its
+ * writes are visible; before it a kernel may only touch what no kernel of a step writes (the
+ * mesh).  pdl_trigger, after the wait, lets the next kernel's blocks start the same way.
+ * Without the launch attribute both do nothing.  Measured together
+ * with the merge of a step's two clock kernels and kGraphSteps (passes of 60 steps on 1,600
+ * triangles and 100 on 200k): 3.36 -> 2.97 ms and 23.6 -> 22.5 ms. */
+DGR_DEV void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+DGR_DEV void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 /* Clock and forcing of one scenario (one mesh of an ensemble; a single mesh is an
  * ensemble of one).  Every scenario advances with its own CFL dt. */
 struct DevClock {
@@ -78,7 +89,7 @@ struct DevClock {
     double tide_amp, tide_period;
     int tide_on;
     int el_off, ed_off; /* first element / edge of the scenario in the flattened mesh */
-    int pad_;
+    int in_step;        /* 1: a step was begun and its end (clock_end_item) is still to be taken */
 };
 
 struct MeshDev {
@@ -181,8 +192,12 @@ DGR_DEV double edge_flux_item(const MeshDev &m, const double *S, const int *wd, 
 {
     double lam = 0.0;
     DevClock *ck = clk + (m.ed_sid ? m.ed_sid[i] : 0);
+    const int el_in = m.e_in[i], el_ex = m.e_ex[i], info = m.e_info[i];
+    if (!COH) {
+        pdl_wait();
+        pdl_trigger();
+    }
     if (!ldm<COH>(&ck->done)) {
-        const int el_in = m.e_in[i], el_ex = m.e_ex[i], info = m.e_info[i];
         const int k_in = info & 3, k_ex = (info >> 2) & 3, bd = (info >> 4) & 7;
         if (!(index_ok(m, el_in, m.ne, KID_EDGE, i) && index_ok(m, el_ex, m.ne, KID_EDGE, i) &&
               index_ok(m, k_in, 3, KID_EDGE, i) && index_ok(m, k_ex, 3, KID_EDGE, i)))
@@ -273,15 +288,15 @@ __global__ void __launch_bounds__(DGR_EDGE_BS, DGR_MINB_EDGE) k_edge_flux(const 
 /* ---------------------------------------------------------------- elements ---- */
 
 /* Gathered numerical fluxes of one element's three edges, sign flipped on the "ex" side
- * (2DCode/2DInnerProducts.c:319-329).  F[variable][local edge]. */
+ * (2DCode/2DInnerProducts.c:319-329).  ee: the element's elem_edge entries;
+ * F[variable][local edge]. */
 template <bool COH>
-DGR_DEV bool gather_flux(const MeshDev &m, const double *flux, int el, double F[3][3])
+DGR_DEV bool gather_flux(const MeshDev &m, const double *flux, int el, const int ee[3], double F[3][3])
 {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const int ee = m.elem_edge[k * m.ldE + el];
-        const int e = ee >> 1;
-        const int side = ee & 1;
+        const int e = ee[k] >> 1;
+        const int side = ee[k] & 1;
         if (!index_ok(m, e, m.nf, KID_ELEMENT, el)) return false;
 #pragma unroll
         for (int v = 0; v < 3; ++v) {
@@ -313,13 +328,18 @@ DGR_DEV void element_item(const MeshDev &m, const double *S, const double *U, co
                           double *out, double *avg, const DevClock *clk, double g, int el)
 {
     const DevClock *ck = clk + (m.el_sid ? m.el_sid[el] : 0);
+    const int ld = m.ldE;
+    const int ee[3] = {m.elem_edge[el], m.elem_edge[ld + el], m.elem_edge[2 * ld + el]};
+    if (!COH) {
+        pdl_wait();
+        pdl_trigger();
+    }
     if (ldm<COH>(&ck->done)) return;
     const double rain = ck->rain;
-    const int ld = m.ldE;
     const double *G = m.geo + geo_offset(el, ld);
     const int gs = geo_stride(ld);
     double F[3][3];
-    if (!gather_flux<COH>(m, flux, el, F)) return;
+    if (!gather_flux<COH>(m, flux, el, ee, F)) return;
     double zr[3], qxr[3], qyr[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -373,6 +393,10 @@ DGR_DEV void node_item(const MeshDev &m, const double *avg, double *bounds, int 
     if (!(index_ok(m, b, 3 * m.ne + 1, KID_NODE, n) && index_ok(m, e, 3 * m.ne + 1, KID_NODE, n) &&
           index_ok(m, e - b, 3 * m.ne + 1, KID_NODE, n)))
         return;
+    if (!COH) {
+        pdl_wait();
+        pdl_trigger();
+    }
     for (int j = b; j < e; ++j) {
         const int el = m.n2e[j];
         if (!index_ok(m, el, m.ne, KID_NODE, n)) return;
@@ -454,9 +478,13 @@ DGR_DEV void limit_item(const MeshDev &m, double *S, const double *bounds, const
                         DevClock *clk, double h0, double velzero, int phase, int *dec_limit, int *dec_pdop, int el)
 {
     DevClock *ck = clk + (m.el_sid ? m.el_sid[el] : 0);
-    if (ldm<COH>(&ck->done)) return;
     const int ld = m.ldE;
     const int nd[3] = {m.el2v[el], m.el2v[ld + el], m.el2v[2 * ld + el]};
+    if (!COH) {
+        pdl_wait();
+        pdl_trigger();
+    }
+    if (ldm<COH>(&ck->done)) return;
     if (!(index_ok(m, nd[0], m.nn, KID_LIMIT, el) && index_ok(m, nd[1], m.nn, KID_LIMIT, el) &&
           index_ok(m, nd[2], m.nn, KID_LIMIT, el)))
         return;
@@ -518,9 +546,25 @@ __global__ void __launch_bounds__(BS, DGR_LIMIT_THREADS_PER_SM / BS) k_limit(con
 
 /* ------------------------------------------------------------------ clock ---- */
 
+/* End of a step: step counter and the pending CFL update, taken by whichever clock kernel
+ * comes next (the next step's, or k_clock_finish).  A scenario whose step just failed stops
+ * here, so its step count is the number of steps that completed. */
+DGR_DEV void clock_end_item(DevClock *c)
+{
+    if (!c->in_step) return;
+    c->in_step = 0;
+    if (c->done) return;
+    if (c->err != ~0ull) {
+        c->done = 1;
+        return;
+    }
+    c->step += 1;
+    c->dt_pending = 1;
+}
+
 /*
  * Start of one step of the device time loop (2DCode/time_evolution.c:311-401), for every
- * scenario: finish the CFL dt of the previous step, stop when time has reached
+ * scenario: take the end of the previous step, finish its CFL dt, stop when time has reached
  * final_time, evaluate the boundary values for this step (boundary_conditions() at the
  * current time), then advance the clock.  One block; thread s owns scenario s's clock,
  * then all threads write the prescribed edges.
@@ -531,6 +575,7 @@ DGR_DEV void clock_begin_body(DevClock *clk, int nscen, const PhysParams &p, con
 {
     for (int s = threadIdx.x; s < nscen; s += blockDim.x) {
         DevClock *c = clk + s;
+        clock_end_item(c);
         if (c->done) continue;
         if (c->dt_pending) {
             const double lam = __longlong_as_double((long long)c->lam_bits[p.stages - 1]);
@@ -548,6 +593,7 @@ DGR_DEV void clock_begin_body(DevClock *clk, int nscen, const PhysParams &p, con
         c->lam_bits[0] = 0;
         c->lam_bits[1] = 0;
         c->lam_bits[2] = 0;
+        c->in_step = 1;
     }
     __syncthreads();
     for (int j = threadIdx.x; j < nbnd; j += blockDim.x) {
@@ -570,27 +616,9 @@ static __global__ void __launch_bounds__(256) k_clock_begin(DevClock *clk, int n
                                                      const int *__restrict__ bnd_sid, int nbnd,
                                                      double *__restrict__ bzeta, double *__restrict__ bqn)
 {
+    pdl_wait();
+    pdl_trigger();
     clock_begin_body(clk, nscen, p, bnd_edges, bnd_type, bnd_sid, nbnd, bzeta, bqn);
-}
-
-/* End of a step: step counters and the pending CFL updates.  A scenario whose step just
- * failed stops here, so its step count is the number of steps that completed. */
-template <bool COH = false>
-DGR_DEV void clock_end_item(DevClock *clk, int s)
-{
-    if (clk[s].done) return;
-    if (ldm<COH>(&clk[s].err) != ~0ull) {
-        clk[s].done = 1;
-        return;
-    }
-    clk[s].step += 1;
-    clk[s].dt_pending = 1;
-}
-
-static __global__ void k_clock_end(DevClock *clk, int nscen)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < nscen) clock_end_item(clk, s);
 }
 
 /* After a run: derive each scenario's next dt so the host sees it. */
@@ -599,6 +627,7 @@ static __global__ void k_clock_finish(DevClock *clk, int nscen, PhysParams p)
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nscen) return;
     DevClock *c = clk + s;
+    clock_end_item(c);
     if (c->dt_pending) {
         const double lam = __longlong_as_double((long long)c->lam_bits[p.stages - 1]);
         double dt = p.cfl * c->min_edge / lam;
@@ -609,15 +638,19 @@ static __global__ void k_clock_finish(DevClock *clk, int nscen, PhysParams p)
 }
 
 /* Gauge values after a step of the device loop: row (step - 1) of the series holds
- * zeta_g = sum_k w[nm g + k] zeta_k(el_g) for the step count of the gauge's scenario (a
- * finished scenario rewrites its last row with the same state). */
+ * zeta_g = sum_k w[nm g + k] zeta_k(el_g) for the step count of the gauge's scenario, the
+ * step whose end is still to be taken included (a finished scenario rewrites its last row
+ * with the same state). */
 static __global__ void k_gauge_record(const double *__restrict__ S, int ld, int nm, int ng, const int *__restrict__ g_el,
                                       const int *__restrict__ g_sid, const double *__restrict__ g_w,
                                       const DevClock *clk, int cap, double *__restrict__ series)
 {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ng) return;
-    const int step = clk[g_sid[g]].step;
+    pdl_wait();
+    pdl_trigger();
+    const DevClock *c = clk + g_sid[g];
+    const int step = c->step + (c->in_step && !c->done && c->err == ~0ull);
     if (step < 1 || step > cap) return;
     const int el = g_el[g];
     double z = g_w[nm * g] * S[el];
@@ -631,6 +664,7 @@ static __global__ void k_clock_set(DevClock *clk, double time, double dt)
     clk->time = time;
     clk->dt = dt;
     clk->done = 0;
+    clk->in_step = 0;
     clk->lam_bits[0] = 0;
     clk->lam_bits[1] = 0;
     clk->lam_bits[2] = 0;
@@ -767,8 +801,6 @@ __global__ void __launch_bounds__(BS, 512 / BS) k_step_fused(const __grid_consta
         if (stage + 1 < stage_end || with_clock)
             if (!grid_barrier(a.bar, a.bar_polls, a.bar_phantom)) return;
     }
-    if (with_clock && blockIdx.x == 0)
-        for (int sc = threadIdx.x; sc < a.nscen; sc += BS) clock_end_item<true>(a.clk, sc);
 }
 
 /* ---------------------------------------------------------------- set-up ---- */

@@ -243,8 +243,10 @@ __global__ void __launch_bounds__(BS, DGR_P2_MINB_EDGE) k_p2_edge(P2Ref ref, Mes
     double lam = 0.0;
     if (valid) {
         DevClock *ck = clk + sid;
+        const int el_in = m.e_in[i], el_ex = m.e_ex[i], info = m.e_info[i];
+        pdl_wait();
+        pdl_trigger();
         if (!ck->done) {
-            const int el_in = m.e_in[i], el_ex = m.e_ex[i], info = m.e_info[i];
             const int k_in = info & 3;
             const int bd = (info >> 4) & 7;
             const double nx = m.e_geo[i], ny = m.e_geo[m.ldF + i];
@@ -298,6 +300,8 @@ __global__ void __launch_bounds__(BS, DGR_P2_MINB_ELEMENT) k_p2_element(P2Ref re
     const int el = blockIdx.x * BS + threadIdx.x;
     if (el >= m.ne) return;
     const DevClock *ck = clk + (m.el_sid ? m.el_sid[el] : 0);
+    pdl_wait();
+    pdl_trigger();
     if (ck->done) return;
     const int ld = m.ldE;
     double s[3][P2_NM];

@@ -144,6 +144,7 @@ static __global__ void __launch_bounds__(256) k_adj_clock_begin(DevClock *clk, i
 {
     const size_t row = (size_t)n * nscen;
     for (int s = threadIdx.x; s < nscen; s += blockDim.x) {
+        clock_end_item(clk + s);
         if (replay) {
             clk[s].dt = dt_hist[row + s];
             clk[s].dt_pending = 0;
