@@ -443,17 +443,6 @@ DGR_HD double pow43(double x)
 #endif
 }
 
-/* x / d for the limiter's redistribution count d in {1, 2, 3} (as a double).  Division
- * by 1 and by 2 are exact (x and x*0.5 are the correctly rounded x/d); only d = 3 needs
- * the full IEEE division. */
-template <class T>
-DGR_HD T div_by_count(const T &x, double d)
-{
-    if (d == 1.0) return x;
-    if (d == 2.0) return x * 0.5;
-    return x / d;
-}
-
 /* RT0 fit F = (a + b x, c + b y) through three normal-flux values (Cramer's rule of
  * 2DCode/2DInnerProducts.c:134-146 and :507-519). */
 template <class T>
