@@ -110,11 +110,49 @@ DGR_HD double div_rcp(double a, double b, double y, bool &ok)
     return a == 0.0 ? q0 : q2;
 }
 
+/* x / 3 as the IEEE division.  One correction of div_rcp with y = RN(1/3) is enough for
+ * every finite x, underflow included: q0 = x y is within two last places of x/3, the
+ * residual x - 3 q0 is then a small multiple of q0's last place, so exact down to the least
+ * subnormal, and x/3 lies a whole number of thirds of a last place from q0, so at least a
+ * sixth away from every rounding midpoint.  A zero keeps its sign, an infinity takes x y.
+ * With div_rcp here, whose range check sent every element whose momentum had underflowed to
+ * a second, plain pass, a 4M coastal step 170 steps in took 2.62 ms (limiter 235 us), with
+ * this 2.55 ms (202 us). */
+DGR_HD double third(double x)
+{
+    const double y = 1.0 / 3;
+    const double q0 = x * y;
+    const double q = fma(fma(-3.0, q0, x), y, q0);
+    return exponent_bits(x) == 0x7ffu ? q0 : copysign(q, x);
+}
+template <class T>
+DGR_HD T third(const T &x) { return x / 3; }
+
 /* whether b may serve as div_rcp's divisor: |b| within [2^-100, 2^100] */
 DGR_HD bool rcp_divisor_ok(double b)
 {
     const unsigned e = exponent_bits(b);
     return e >= 1023u - 100u && e <= 1023u + 100u;
+}
+
+/* a0 / b and a1 / b as the IEEE divisions: doubles through one reciprocal, plain where that
+ * is not valid */
+DGR_HD void quotient_pair(double a0, double a1, double b, double &q0, double &q1)
+{
+    const double y = 1.0 / b;
+    bool ok = rcp_divisor_ok(b);
+    q0 = div_rcp(a0, b, y, ok);
+    q1 = div_rcp(a1, b, y, ok);
+    if (!ok) {
+        q0 = a0 / b;
+        q1 = a1 / b;
+    }
+}
+template <class T>
+DGR_HD void quotient_pair(const T &a0, const T &a1, const T &b, T &q0, T &q1)
+{
+    q0 = a0 / b;
+    q1 = a1 / b;
 }
 
 /* rt0_fit below with its three divisions by dM taken through div_rcp (y = 1/dM) */

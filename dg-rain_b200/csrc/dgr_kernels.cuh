@@ -459,21 +459,7 @@ static __global__ void __launch_bounds__(256) k_wd_status(MeshDev m, const doubl
  * wet/dry status (2DCode/wetDry2D.c:16-60) that the reference calls next.  wd_in is the
  * status the element had; the new status goes to wd_out.
  */
-template <bool LIMIT, bool PDOP, bool STATUS, bool COH = false, bool RCP = false>
-DGR_DEV void limit_item(const MeshDev &m, double *S, const double *bounds, const int *wd_in, int *wd_out,
-                        DevClock *clk, double h0, double velzero, int phase, int *dec_limit, int *dec_pdop, int el);
-
-/* an element where the shared reciprocals are not valid, with plain divisions, kept out of
- * line: its state is still untouched */
-template <bool LIMIT, bool PDOP, bool STATUS>
-__device__ __noinline__ void limit_item_plain(const MeshDev &m, double *S, const double *bounds, const int *wd_in,
-                                              int *wd_out, DevClock *clk, double h0, double velzero, int phase,
-                                              int *dec_limit, int *dec_pdop, int el)
-{
-    limit_item<LIMIT, PDOP, STATUS>(m, S, bounds, wd_in, wd_out, clk, h0, velzero, phase, dec_limit, dec_pdop, el);
-}
-
-template <bool LIMIT, bool PDOP, bool STATUS, bool COH, bool RCP>
+template <bool LIMIT, bool PDOP, bool STATUS, bool COH = false>
 DGR_DEV void limit_item(const MeshDev &m, double *S, const double *bounds, const int *wd_in, int *wd_out,
                         DevClock *clk, double h0, double velzero, int phase, int *dec_limit, int *dec_pdop, int el)
 {
@@ -499,17 +485,7 @@ DGR_DEV void limit_item(const MeshDev &m, double *S, const double *bounds, const
         return ldm<COH>(&bounds[(3 * is_min + v) * lb + nd[k]]);
     };
     LimitDecisions dec;
-    RcpDiv dv;
-    if constexpr (RCP) {
-        limit_core<LIMIT, PDOP, double, decltype(bnd), false, RcpDiv>(w, bnd, zn, h0, velzero, dec, nullptr, &dv);
-        if (!dv.ok) {
-            limit_item_plain<LIMIT, PDOP, STATUS>(m, S, bounds, wd_in, wd_out, clk, h0, velzero, phase, dec_limit,
-                                                  dec_pdop, el);
-            return;
-        }
-    } else {
-        limit_core<LIMIT, PDOP, double>(w, bnd, zn, h0, velzero, dec);
-    }
+    limit_core<LIMIT, PDOP, double>(w, bnd, zn, h0, velzero, dec);
     if (LIMIT && dec_limit) dec_limit[el] = dec.modify;
     if (PDOP) {
         if (dec.code) atomicMin(&ck->err, err_key(ldm<COH>(&ck->step), phase, dec.code, el - ck->el_off));
@@ -519,16 +495,7 @@ DGR_DEV void limit_item(const MeshDev &m, double *S, const double *bounds, const
     for (int v = 0; v < 3; ++v)
 #pragma unroll
         for (int k = 0; k < 3; ++k) S[(3 * v + k) * ld + el] = w[v][k];
-    if (STATUS) {
-        if constexpr (RCP) {
-            const int st = wd_status(w[0], zn, ldm<COH>(&wd_in[el]), h0, &dv);
-            /* the element's state is written: a status that needs the plain division is
-             * taken with it here (one division, so inline) */
-            wd_out[el] = dv.ok ? st : wd_status(w[0], zn, ldm<COH>(&wd_in[el]), h0);
-        } else {
-            wd_out[el] = wd_status(w[0], zn, ldm<COH>(&wd_in[el]), h0);
-        }
-    }
+    if (STATUS) wd_out[el] = wd_status(w[0], zn, ldm<COH>(&wd_in[el]), h0);
 }
 
 template <bool LIMIT, bool PDOP, bool STATUS, int BS>
@@ -540,8 +507,7 @@ __global__ void __launch_bounds__(BS, DGR_LIMIT_THREADS_PER_SM / BS) k_limit(con
 {
     const int el = blockIdx.x * BS + threadIdx.x;
     if (el < m.ne)
-        limit_item<LIMIT, PDOP, STATUS, false, true>(m, S, bounds, wd_in, wd_out, clk, h0, velzero, phase, dec_limit,
-                                                     dec_pdop, el);
+        limit_item<LIMIT, PDOP, STATUS>(m, S, bounds, wd_in, wd_out, clk, h0, velzero, phase, dec_limit, dec_pdop, el);
 }
 
 /* ------------------------------------------------------------------ clock ---- */

@@ -433,7 +433,7 @@ DGR_HD void element_core(const T F[3][3], const T zr[3], const T qxr[3], const T
     if constexpr (RCP) { /* the means' divisions by 3 through the reciprocal RN(1/3) */
         bool ok_avg = true;
 #pragma unroll
-        for (int v = 0; v < 3; ++v) avg[v] = div_rcp(w[v][0] + w[v][1] + w[v][2], 3.0, 1.0 / 3, ok_avg);
+        for (int v = 0; v < 3; ++v) avg[v] = third(w[v][0] + w[v][1] + w[v][2]);
         *rcp_ok = ok && ok_avg;
     } else {
 #pragma unroll
@@ -464,19 +464,10 @@ struct LimitTrace {
  * at the element's vertex k; zn are the vertex depths.  With TRACE the limiter's path is
  * recorded in *trace (values are unaffected).
  */
-template <bool LIMIT, bool PDOP, class T, class Bnd, bool TRACE = false, class Div = PlainDiv>
+template <bool LIMIT, bool PDOP, class T, class Bnd, bool TRACE = false>
 DGR_HD void limit_core(T w[3][3], const Bnd &bnd, const T zn[3], double h0, double velzero, LimitDecisions &dec,
-                       LimitTrace *trace = nullptr, Div *dv = nullptr)
+                       LimitTrace *trace = nullptr)
 {
-    /* divisions by 3 and by the vertex depths: plain, or (Div = RcpDiv) through shared
-     * reciprocals (div_rcp, the same bits; dv->ok reports where that is not valid) */
-    constexpr bool rcp = std::is_same<Div, RcpDiv>::value;
-    const auto div3 = [&](const T &x) -> T {
-        if constexpr (rcp)
-            return dv->div(x, RcpDiv::By{3.0, 1.0 / 3});
-        else
-            return x / 3;
-    };
     dec.modify = 0;
     dec.mass_branch = 0;
     dec.mom_branch = 0;
@@ -505,7 +496,7 @@ DGR_HD void limit_core(T w[3][3], const Bnd &bnd, const T zn[3], double h0, doub
                     vmax[k] = bnd(v, k, 0);
                     vmin[k] = bnd(v, k, 1);
                 }
-                const T avg = div3(w1 + w2 + w3);
+                const T avg = third(w1 + w2 + w3);
                 unsigned long long tb = 0;
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
@@ -521,7 +512,7 @@ DGR_HD void limit_core(T w[3][3], const Bnd &bnd, const T zn[3], double h0, doub
                  * the instruction cache (measured: 8 % off the limiter kernel rolled) */
 #pragma unroll 1
                 for (int ll = 0; ll < 3; ++ll) { /* :254-299 */
-                    const T sumloc = div3(vx[0] + vx[1] + vx[2]);
+                    const T sumloc = third(vx[0] + vx[1] + vx[2]);
                     T sumdiff = (sumloc - avg) * 3;
                     const int sd = sgn(sumdiff);
                     if (!TRACE && sd == 0) break; /* nothing left to move: later passes change nothing */
@@ -539,7 +530,7 @@ DGR_HD void limit_core(T w[3][3], const Bnd &bnd, const T zn[3], double h0, doub
                         if (up[k]) {
                             redfac = sumdiff * sdd;
                             if (k < 2 && left == 2) redfac = redfac * 0.5;
-                            if (k == 0 && left == 3) redfac = div3(redfac);
+                            if (k == 0 && left == 3) redfac = third(redfac);
                             --left;
                         } else {
                             redfac = 0;
@@ -578,7 +569,7 @@ DGR_HD void limit_core(T w[3][3], const Bnd &bnd, const T zn[3], double h0, doub
         T ht[3] = {mh0 - mh1 + mh2, mh0 + mh1 - mh2, -mh0 + mh1 + mh2};
         int code = 0;
         if (ht[0] <= h0 || ht[1] <= h0 || ht[2] <= h0) { /* :93-156 */
-            const T avg_h = div3(ht[0] + ht[1] + ht[2]);
+            const T avg_h = third(ht[0] + ht[1] + ht[2]);
             if (avg_h <= h0) {
                 dec.mass_branch = 1;
                 ht[0] = avg_h;
@@ -632,14 +623,7 @@ DGR_HD void limit_core(T w[3][3], const Bnd &bnd, const T zn[3], double h0, doub
                 T u[3], vv[3];
 #pragma unroll
                 for (int i = 0; i < 3; ++i) {
-                    if constexpr (rcp) {
-                        const auto by_h = dv->by(ht[i]);
-                        u[i] = dv->div(qxe[i], by_h);
-                        vv[i] = dv->div(qye[i], by_h);
-                    } else {
-                        u[i] = qxe[i] / ht[i];
-                        vv[i] = qye[i] / ht[i];
-                    }
+                    quotient_pair(qxe[i], qye[i], ht[i], u[i], vv[i]);
                 }
                 int npos = 0;
                 T delu = 0, delv = 0;
@@ -676,11 +660,11 @@ DGR_HD void limit_core(T w[3][3], const Bnd &bnd, const T zn[3], double h0, doub
 DGR_HD int big_theta(double a) { return a > 0 ? 1 : 0; }
 
 /* wetDryStatus2D for one element (2DCode/wetDry2D.c:18-57). */
-DGR_HD int wd_status(const double mz[3], const double zn[3], int wd_prev, double h0, RcpDiv *dv = nullptr)
+DGR_HD int wd_status(const double mz[3], const double zn[3], int wd_prev, double h0)
 {
     const double zv[3] = {mz[0] - mz[1] + mz[2], mz[0] + mz[1] - mz[2], -mz[0] + mz[1] + mz[2]};
     const double h[3] = {zv[0] + zn[0], zv[1] + zn[1], zv[2] + zn[2]};
-    const double avg_h = dv ? dv->div(h[0] + h[1] + h[2], RcpDiv::By{3.0, 1.0 / 3}) : (h[0] + h[1] + h[2]) / 3;
+    const double avg_h = third(h[0] + h[1] + h[2]);
     int imax = 0;
     double hmax = h[0];
     if (h[1] > hmax) { imax = 1; hmax = h[1]; }
