@@ -213,6 +213,59 @@ static int upload_concat(cudaStream_t s, T *dst, int nscen, const T *const *src,
     return DGR_OK;
 }
 
+/* One shared-memory carveout for the p = 1 step's kernels: what four resident blocks of
+ * k_edge_flux need.  An SM changes its carveout only when it is empty, so with the driver's
+ * choice per kernel (least for the others) no block of the next kernel starts while the edge
+ * kernel or the one before it drains: 24k triangles 59.6 against 57.4 us per step, 200k 168.7
+ * against 166.5; the whole of it taken from L1 costs more (24k 62.2, 200k 195). */
+static void set_carveouts(const dgr_ctx *c)
+{
+    if (c->p.order != 1) return;
+    const auto set = [](auto *kernel) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 40);
+    };
+    const auto edge = [&](auto wd, auto ft) {
+        if (c->nscen > 1)
+            set(k_edge_flux<decltype(wd)::value, decltype(ft)::value, true>);
+        else
+            set(k_edge_flux<decltype(wd)::value, decltype(ft)::value, false>);
+    };
+    const auto edges = [&](auto wd) {
+        if (c->p.flux == 1)
+            edge(wd, std::integral_constant<int, 1>());
+        else if (c->p.flux == 2)
+            edge(wd, std::integral_constant<int, 2>());
+        else
+            edge(wd, std::integral_constant<int, 0>());
+    };
+    const auto items = [&](auto bs) {
+        constexpr int BS = decltype(bs)::value;
+        set(k_element<MODE_STAGE1, BS>);
+        if (c->p.rk_stages == 3) {
+            set(k_element<MODE_RK3_2, BS>);
+            set(k_element<MODE_RK3_3, BS>);
+        } else {
+            set(k_element<MODE_STAGE2, BS>);
+        }
+        if (c->p.wet_dry)
+            set(k_limit<true, true, true, BS>);
+        else
+            set(k_limit<true, false, false, BS>);
+    };
+    if (c->p.wet_dry)
+        edges(std::true_type());
+    else
+        edges(std::false_type());
+    if (c->bs == 64)
+        items(std::integral_constant<int, 64>());
+    else if (c->bs == 256)
+        items(std::integral_constant<int, 256>());
+    else
+        items(std::integral_constant<int, 128>());
+    set(k_node_bounds);
+    set(k_clock_begin);
+}
+
 static int create_impl(int nscen, const dgr_mesh_view *views, const dgr_scenario_params *sp, const dgr_params *params,
                        dgr_ctx **out)
 {
@@ -474,6 +527,7 @@ static int create_impl(int nscen, const dgr_mesh_view *views, const dgr_scenario
     TRYC(cudaMemcpy(c->wdC, wd.data(), ne * 4, cudaMemcpyHostToDevice));
     c->wd_fresh = 0;
     c->wd_stepped = 0;
+    set_carveouts(c);
     *out = c;
     return DGR_OK;
 }
@@ -544,6 +598,7 @@ extern "C" int dgr_set_params(dgr_ctx *c, const dgr_params *p)
         c->wd_stepped = 0;
         c->wd_fresh = 0;
         c->p.rk_stages = stages;
+        set_carveouts(c);
     }
     if (c->nscen == 1) { /* a single mesh takes its forcing from the run parameters */
         int r = read_clock(c);
@@ -782,8 +837,9 @@ template <bool WD, int FT>
 static void launch_edge_ft(dgr_ctx *c, const double *S, const int *wd, int lam_slot, int phase)
 {
     const MeshDev m = mesh_dev(c);
-    launch_dep(k_edge_flux<WD, FT>, blocks(c->nf, DGR_EDGE_BS), DGR_EDGE_BS, c->stream, m, S, wd, c->bzeta, c->bqn, c->flux, c->clk,
-                                                                   lam_slot, phase, c->p.g);
+    const unsigned grid = std::min(blocks(c->nf, DGR_EDGE_BS), (unsigned)(c->num_sms * DGR_MINB_EDGE));
+    launch_dep(c->ed_sid ? k_edge_flux<WD, FT, true> : k_edge_flux<WD, FT, false>, grid, DGR_EDGE_BS, c->stream, m, S, wd,
+               c->bzeta, c->bqn, c->flux, c->clk, lam_slot, phase, c->p.g);
 }
 
 /* the edge kernel compiled for the context's wet/dry mode and numerical flux */
@@ -1367,6 +1423,7 @@ extern "C" int dgr_set_schedule(dgr_ctx *c, int block_size, int fusion)
     if (c->p.order == 2 && fusion != 0) return DGR_ERR_INVALID; /* the p = 2 step has no fused kernel */
     c->bs = block_size;
     c->fusion = fusion;
+    set_carveouts(c);
     drop_graph(c);
     return DGR_OK;
 }
@@ -1410,6 +1467,7 @@ static int autotune_trials(dgr_ctx *c, int trial_steps, double *saveU, int *save
         for (int f = 0; f < (c->p.order == 2 ? 1 : 3); ++f) {
             c->bs = bss[b];
             c->fusion = f;
+            set_carveouts(c);
             drop_graph(c);
             for (int k = 0; k < c->nscen; ++k) {
                 t[k] = clk0[k].time;
@@ -1466,6 +1524,7 @@ extern "C" int dgr_autotune(dgr_ctx *c, int trial_steps, int *block_size, int *f
     const cudaError_t e3 = cudaStreamSynchronize(s);
     c->bs = best_bs;
     c->fusion = best_f;
+    set_carveouts(c);
     drop_graph(c);
     if (rc) return rc;
     CK(e1);

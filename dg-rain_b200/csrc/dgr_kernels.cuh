@@ -23,17 +23,17 @@
 #include "dgr_forcing.h"
 #include "dgr_scheme.cuh"
 
-/* Threads per block of the edge kernel, and the minimum resident blocks per SM requested
- * from the compiler for it (register cap 65536 / (DGR_EDGE_BS x blocks) = 85, so 80);
- * chosen by measurement (4,000,000 triangles: 0.332 ms per launch in blocks of 128, 0.338
- * in blocks of 64, 0.352 in blocks of 256), overridable at build time.  The element
+/* Threads per block of the edge kernel, and its resident blocks per SM (register cap 65536 /
+ * (DGR_EDGE_BS x blocks) = 128); chosen by measurement with the tiles of k_edge_flux
+ * (step at 4M triangles: 2.154 ms in four blocks of 128, 2.160 in three, 2.214 in five, 2.289
+ * in six, 2.168 in eight blocks of 64), overridable at build time.  The element
  * kernels are capped at 128 registers and the limiter kernels at 64
  * (DGR_ELEMENT_THREADS_PER_SM and DGR_LIMIT_THREADS_PER_SM below). */
 #ifndef DGR_EDGE_BS
 #define DGR_EDGE_BS 128
 #endif
 #ifndef DGR_MINB_EDGE
-#define DGR_MINB_EDGE (768 / DGR_EDGE_BS)
+#define DGR_MINB_EDGE (512 / DGR_EDGE_BS)
 #endif
 /* Resident threads per SM requested for the limiter kernel (register cap 65536 / this);
  * chosen by measurement (1024: 64 registers, 0.244 ms at 4M triangles; 768: 80 registers,
@@ -168,10 +168,10 @@ DGR_DEV void prefetch_geometry(const MeshDev &m, int base, int n)
 /* One edge (2DCode/compute2DL.c:17-331): traces, ghost state, Roe flux(es); stores Fhat.n
  * for both sides and returns the edge's max wave speed (0 for a finished scenario).
  * FT: the numerical flux as a compile-time constant (0 Roe, 1 LLF, 2 HLLC), or -1 to take
- * it from the mesh at run time.  RCP: the Roe flux's divisions share one reciprocal per
- * divisor (RcpDiv, the same bits); an edge where that is not valid is redone by
+ * it from the mesh at run time.  RCP (k_edge_flux): the Roe flux's divisions share one
+ * reciprocal per divisor (RcpDiv, the same bits); an edge where that is not valid is redone by
  * edge_item_plain (plain divisions, kept out of line). */
-template <bool WD, bool COH = false, int FT = -1, bool RCP = false>
+template <bool WD, bool COH = false, int FT = -1>
 DGR_DEV double edge_flux_item(const MeshDev &m, const double *S, const int *wd, const double *bzeta,
                               const double *bqn, double *flux, DevClock *clk, int phase, double g, int i);
 
@@ -186,59 +186,61 @@ __device__ __noinline__ double edge_item_plain(const MeshDev &m, const double *S
     return edge_flux_item<WD, false, FT>(m, S, wd, bzeta, bqn, flux, clk, phase, g, i);
 }
 
+/* The edge from its traces on: (zi, qxi, qyi) of the in side, (ze, qxe, qye) of the other side
+ * (of the in side itself at a wall), the sides' wet/dry flags. */
 template <bool WD, bool COH, int FT, bool RCP>
+DGR_DEV double edge_from_traces(const MeshDev &m, const double *S, const int *wd, const double *bzeta,
+                                const double *bqn, double *flux, DevClock *clk, DevClock *ck, int phase, double g,
+                                int i, int bd, bool wall, double nx, double ny, double z_edge, double zi, double qxi,
+                                double qyi, double ze, double qxe, double qye, int wdi, int wde)
+{
+    if (bd)
+        ghost_state<double>(bd, nx, ny, zi, qxi, qyi, ldm<COH>(&bzeta[i]), ldm<COH>(&bqn[i]), 0.0, ze, qxe, qye);
+    else if (wall)
+        ghost_state<double>(0, nx, ny, zi, qxi, qyi, 0.0, 0.0, ze, ze, qxe, qye);
+    double fin[3], fex[3], lam;
+    int code;
+    if constexpr (RCP) {
+        RcpDiv dv;
+        lam = flux_core<double, WD, RcpDiv>(zi, qxi, qyi, ze, qxe, qye, z_edge, nx, ny, wdi, wde, g, fin, fex, code,
+                                            FT >= 0 ? FT : m.flux, &dv);
+        if (!dv.ok) return edge_item_plain<WD, FT>(m, S, wd, bzeta, bqn, flux, clk, phase, g, i);
+    } else {
+        lam = flux_core<double, WD>(zi, qxi, qyi, ze, qxe, qye, z_edge, nx, ny, wdi, wde, g, fin, fex, code,
+                                    FT >= 0 ? FT : m.flux);
+    }
+    if (code) atomicMin(&ck->err, err_key(ldm<COH>(&ck->step), phase, code, i - ck->ed_off));
+    const int lf = m.ldF;
+    flux[i] = fin[0];
+    flux[lf + i] = fin[1];
+    flux[2 * lf + i] = fin[2];
+    flux[3 * lf + i] = fex[0];
+    flux[4 * lf + i] = fex[1];
+    flux[5 * lf + i] = fex[2];
+    return lam >= 0.0 ? lam : 0.0; /* NaN speeds are reported through the flux check */
+}
+
+DGR_DEV bool edge_indices_ok(const MeshDev &m, int i, int el_in, int el_ex, int info)
+{
+    return index_ok(m, el_in, m.ne, KID_EDGE, i) && index_ok(m, el_ex, m.ne, KID_EDGE, i) &&
+           index_ok(m, info & 3, 3, KID_EDGE, i) && index_ok(m, (info >> 2) & 3, 3, KID_EDGE, i);
+}
+
+template <bool WD, bool COH, int FT>
 DGR_DEV double edge_flux_item(const MeshDev &m, const double *S, const int *wd, const double *bzeta,
                               const double *bqn, double *flux, DevClock *clk, int phase, double g, int i)
 {
-    double lam = 0.0;
     DevClock *ck = clk + (m.ed_sid ? m.ed_sid[i] : 0);
+    if (ldm<COH>(&ck->done)) return 0.0;
     const int el_in = m.e_in[i], el_ex = m.e_ex[i], info = m.e_info[i];
-    if (!COH) {
-        pdl_wait();
-        pdl_trigger();
-    }
-    if (!ldm<COH>(&ck->done)) {
-        const int k_in = info & 3, k_ex = (info >> 2) & 3, bd = (info >> 4) & 7;
-        if (!(index_ok(m, el_in, m.ne, KID_EDGE, i) && index_ok(m, el_ex, m.ne, KID_EDGE, i) &&
-              index_ok(m, k_in, 3, KID_EDGE, i) && index_ok(m, k_ex, 3, KID_EDGE, i)))
-            return 0.0;
-        const double nx = m.e_geo[i], ny = m.e_geo[m.ldF + i], z_edge = m.e_geo[2 * m.ldF + i];
-        const int ld = m.ldE;
-        const double zi = ldm<COH>(&S[k_in * ld + el_in]), qxi = ldm<COH>(&S[(3 + k_in) * ld + el_in]),
-                     qyi = ldm<COH>(&S[(6 + k_in) * ld + el_in]);
-        double ze, qxe, qye;
-        if (bd)
-            ghost_state<double>(bd, nx, ny, zi, qxi, qyi, ldm<COH>(&bzeta[i]), ldm<COH>(&bqn[i]), 0.0, ze, qxe, qye);
-        else if (el_in == el_ex)
-            ghost_state<double>(0, nx, ny, zi, qxi, qyi, 0.0, 0.0, ldm<COH>(&S[k_ex * ld + el_ex]), ze, qxe, qye);
-        else {
-            ze = ldm<COH>(&S[k_ex * ld + el_ex]);
-            qxe = ldm<COH>(&S[(3 + k_ex) * ld + el_ex]);
-            qye = ldm<COH>(&S[(6 + k_ex) * ld + el_ex]);
-        }
-        const int wdi = WD ? ldm<COH>(&wd[el_in]) : 1, wde = WD ? ldm<COH>(&wd[el_ex]) : 1;
-        double fin[3], fex[3];
-        int code;
-        if constexpr (RCP) {
-            RcpDiv dv;
-            lam = flux_core<double, WD, RcpDiv>(zi, qxi, qyi, ze, qxe, qye, z_edge, nx, ny, wdi, wde, g, fin, fex,
-                                                code, FT >= 0 ? FT : m.flux, &dv);
-            if (!dv.ok) return edge_item_plain<WD, FT>(m, S, wd, bzeta, bqn, flux, clk, phase, g, i);
-        } else {
-            lam = flux_core<double, WD>(zi, qxi, qyi, ze, qxe, qye, z_edge, nx, ny, wdi, wde, g, fin, fex, code,
-                                        FT >= 0 ? FT : m.flux);
-        }
-        if (code) atomicMin(&ck->err, err_key(ldm<COH>(&ck->step), phase, code, i - ck->ed_off));
-        const int lf = m.ldF;
-        flux[i] = fin[0];
-        flux[lf + i] = fin[1];
-        flux[2 * lf + i] = fin[2];
-        flux[3 * lf + i] = fex[0];
-        flux[4 * lf + i] = fex[1];
-        flux[5 * lf + i] = fex[2];
-        if (!(lam >= 0.0)) lam = 0.0; /* NaN speeds are reported through the flux check */
-    }
-    return lam;
+    if (!edge_indices_ok(m, i, el_in, el_ex, info)) return 0.0;
+    const int k_in = info & 3, k_ex = (info >> 2) & 3, ld = m.ldE;
+    const auto st = [S, ld](int plane, int el) { return ldm<COH>(&S[plane * ld + el]); };
+    return edge_from_traces<WD, COH, FT, false>(
+        m, S, wd, bzeta, bqn, flux, clk, ck, phase, g, i, (info >> 4) & 7, el_in == el_ex, m.e_geo[i],
+        m.e_geo[m.ldF + i], m.e_geo[2 * m.ldF + i], st(k_in, el_in), st(3 + k_in, el_in), st(6 + k_in, el_in),
+        st(k_ex, el_ex), st(3 + k_ex, el_ex), st(6 + k_ex, el_ex), WD ? ldm<COH>(&wd[el_in]) : 1,
+        WD ? ldm<COH>(&wd[el_ex]) : 1);
 }
 
 /* Max of the wave speed per scenario: one atomic per block when the block's edges all
@@ -269,20 +271,102 @@ DGR_DEV void block_max_speed(double lam, int sid, bool valid, DevClock *clk, int
     }
 }
 
-template <bool WD, int FT>
-__global__ void __launch_bounds__(DGR_EDGE_BS, DGR_MINB_EDGE) k_edge_flux(const __grid_constant__ MeshDev m, const double *__restrict__ S,
-                                                                  const int *__restrict__ wd,
-                                                                  const double *__restrict__ bzeta,
-                                                                  const double *__restrict__ bqn,
-                                                                  double *__restrict__ flux, DevClock *clk,
-                                                                  int lam_slot, int phase, double g)
+DGR_DEV void copy_async8(double *dst, const double *src)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < m.nf;
-    const int sid = (valid && m.ed_sid) ? m.ed_sid[i] : 0;
-    const double lam =
-        valid ? edge_flux_item<WD, false, FT, FT == 0>(m, S, wd, bzeta, bqn, flux, clk, phase, g, i) : 0.0;
-    block_max_speed(lam, sid, valid, clk, lam_slot);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(__cvta_generic_to_global(src))
+                 : "memory");
+}
+DGR_DEV void copy_async4(int *dst, const int *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(__cvta_generic_to_global(src))
+                 : "memory");
+}
+
+/* All edges, in tiles of BS: at most as many blocks as are resident, each taking several
+ * tiles, with the next tile's traces, geometry and flags on their way to shared memory
+ * (cp.async, every thread its own edge's: no barrier) and the indices of the one after in
+ * registers while a tile is computed.  The kernel is bound by FP64 dependency chains and was
+ * waiting for the gathers behind the indices as much (4.3 cycles per issue); with them in
+ * flight 16 warps per SM at 128 registers, without most spills, beat 24 at 80.  Against one
+ * edge per thread, per step: 4M triangles 2.197 -> 2.137 ms, 200k 171 -> 166 us, RK3 HLLC 91k
+ * 114 -> 111, ensemble of 32 (0.9M) 482 -> 469, 24k 58.1 -> 57.9, 1,600 45.1 -> 45.0. */
+template <bool WD, int FT, bool ENS>
+__global__ void __launch_bounds__(DGR_EDGE_BS, DGR_MINB_EDGE)
+    k_edge_flux(const __grid_constant__ MeshDev m, const double *__restrict__ S, const int *__restrict__ wd,
+                const double *__restrict__ bzeta, const double *__restrict__ bqn, double *__restrict__ flux,
+                DevClock *clk, int lam_slot, int phase, double g)
+{
+    constexpr int BS = DGR_EDGE_BS;
+    __shared__ double tr[2][9][BS];
+    __shared__ int fl[2][2][BS];
+    const int t = threadIdx.x, ld = m.ldE, lf = m.ldF;
+    /* a single mesh deals the tiles out in turn; in an ensemble (ENS) a block takes
+     * consecutive ones, which mostly belong to one scenario */
+    const int mine = ENS ? ((m.nf + BS - 1) / BS + gridDim.x - 1) / gridDim.x * BS : BS;
+    const int begin = blockIdx.x * mine, stride = ENS ? BS : gridDim.x * BS;
+    const int end = ENS ? min(begin + mine, m.nf) : m.nf;
+    int i = begin + t;
+    int el_in = 0, el_ex = 0, info = -1; /* of the edge to fetch next */
+    const auto indices = [&](int j) {
+        info = -1;
+        if (j < end) {
+            el_in = m.e_in[j];
+            el_ex = m.e_ex[j];
+            info = m.e_info[j];
+            if (!edge_indices_ok(m, j, el_in, el_ex, info)) info = -1;
+        }
+    };
+    /* starts the copies of edge j's data into stage b; what the flux still needs of the
+     * indices: boundary type and wall, or -1 for no edge */
+    const auto fetch = [&](int j, int b) {
+        if (info < 0) return -1;
+        const int k_in = info & 3, k_ex = (info >> 2) & 3;
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+            copy_async8(&tr[b][v][t], &S[(3 * v + k_in) * ld + el_in]);
+            copy_async8(&tr[b][3 + v][t], &S[(3 * v + k_ex) * ld + el_ex]);
+            copy_async8(&tr[b][6 + v][t], &m.e_geo[(size_t)v * lf + j]);
+        }
+        if (WD) {
+            copy_async4(&fl[b][0][t], &wd[el_in]);
+            copy_async4(&fl[b][1][t], &wd[el_ex]);
+        }
+        return ((info >> 4) & 7) | (el_in == el_ex ? 8 : 0);
+    };
+    indices(i);
+    pdl_wait();
+    pdl_trigger();
+    if (!ENS && clk->done) return;
+    int kind = fetch(i, 0), b = 0;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    indices(i + stride);
+    double lam_all = 0.0; /* of scenario sid, until the thread meets another one */
+    int sid = 0;
+    for (int base = begin; base < end; base += stride, i += stride, b ^= 1) {
+        const int next = fetch(i + stride, b ^ 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        indices(i + 2 * stride);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        if (kind >= 0) {
+            if (ENS && m.ed_sid[i] != sid) {
+                if (lam_all > 0.0)
+                    atomicMax(&clk[sid].lam_bits[lam_slot], (unsigned long long)__double_as_longlong(lam_all));
+                lam_all = 0.0;
+                sid = m.ed_sid[i];
+            }
+            DevClock *ck = clk + sid;
+            if (!(ENS && ck->done))
+                lam_all = fmax(lam_all,
+                               edge_from_traces<WD, false, FT, FT == 0>(
+                                   m, S, wd, bzeta, bqn, flux, clk, ck, phase, g, i, kind & 7, (kind & 8) != 0,
+                                   tr[b][6][t], tr[b][7][t], tr[b][8][t], tr[b][0][t], tr[b][1][t], tr[b][2][t],
+                                   tr[b][3][t], tr[b][4][t], tr[b][5][t], WD ? fl[b][0][t] : 1, WD ? fl[b][1][t] : 1));
+        }
+        kind = next;
+    }
+    block_max_speed(lam_all, sid, true, clk, lam_slot);
 }
 
 /* ---------------------------------------------------------------- elements ---- */
