@@ -147,6 +147,7 @@ static P2Ref make_p2_ref()
         p2_basis(r, sv, R.phi[q], R.dr[q], R.ds[q]);
         for (int m = 0; m < P2_NM; ++m) R.mass[m] += 2.0 * W[q] * R.phi[q][m] * R.phi[q][m];
     }
+    for (int m = 0; m < P2_NM; ++m) R.imass[m] = 1.0 / R.mass[m];
     const double g3 = sqrt(3.0 / 5);
     const double te[P2_NGP] = {-g3, 0.0, g3}, wg[P2_NGP] = {5.0 / 9, 8.0 / 9, 5.0 / 9};
     for (int gp = 0; gp < P2_NGP; ++gp) {

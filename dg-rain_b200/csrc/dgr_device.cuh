@@ -41,6 +41,9 @@ DGR_HD T rmax(const T &a, const T &b) { return (a > b) ? a : b; }
 template <class T>
 DGR_HD T rmin(const T &a, const T &b) { return (a < b) ? a : b; }
 
+/* a b + c rounded once (the p = 2 cores; the two-lane overloads live with their types) */
+DGR_HD double muladd(double a, double b, double c) { return fma(a, b, c); }
+
 /* value of a scalar (decisions are taken on values; the dual-number overload lives with
  * the dual type) */
 DGR_HD double val(double x) { return x; }

@@ -55,6 +55,13 @@ DGR_HD Dual operator/(double a, const Dual &b)
     const double q = a / b.v;
     return Dual(q, -q * b.d / b.v);
 }
+/* the value rounded once, as the double muladd */
+DGR_HD Dual muladd(const Dual &a, const Dual &b, const Dual &c)
+{
+    return Dual(dgr::muladd(a.v, b.v, c.v), a.d * b.v + a.v * b.d + c.d);
+}
+DGR_HD Dual muladd(double a, const Dual &b, const Dual &c) { return Dual(dgr::muladd(a, b.v, c.v), a * b.d + c.d); }
+DGR_HD Dual muladd(const Dual &a, double b, const Dual &c) { return muladd(b, a, c); }
 DGR_HD Dual &operator+=(Dual &a, const Dual &b) { return a = a + b; }
 DGR_HD Dual &operator-=(Dual &a, const Dual &b) { return a = a - b; }
 
@@ -137,6 +144,15 @@ DGR_HD Pert operator*(double a, const Pert &b) { return Pert(a * b.v, a * b.p); 
 DGR_HD Pert operator/(const Pert &a, const Pert &b) { return Pert(a.v / b.v, a.p / b.p); }
 DGR_HD Pert operator/(const Pert &a, double b) { return Pert(a.v / b, a.p / b); }
 DGR_HD Pert operator/(double a, const Pert &b) { return Pert(a / b.v, a / b.p); }
+DGR_HD Pert muladd(const Pert &a, const Pert &b, const Pert &c)
+{
+    return Pert(dgr::muladd(a.v, b.v, c.v), dgr::muladd(a.p, b.p, c.p));
+}
+DGR_HD Pert muladd(double a, const Pert &b, const Pert &c)
+{
+    return Pert(dgr::muladd(a, b.v, c.v), dgr::muladd(a, b.p, c.p));
+}
+DGR_HD Pert muladd(const Pert &a, double b, const Pert &c) { return muladd(b, a, c); }
 DGR_HD Pert &operator+=(Pert &a, const Pert &b) { return a = a + b; }
 DGR_HD Pert &operator-=(Pert &a, const Pert &b) { return a = a - b; }
 

@@ -18,6 +18,13 @@
  * numerical flux is the Roe flux of 2DCode (roe_flux) at each edge Gauss point.  The depth
  * is linear per element (the node depths), which keeps a lake at rest exactly at rest.
  * No limiter and no wet/dry treatment: the p = 2 step is for flows that stay wet.
+ *
+ * No reference fixes the bits here, so the sums over modes and points are fused multiply-adds
+ * (the library is otherwise built without contraction).  Both kernels are bound by FP64
+ * dependency chains: with those sums, the flux's components along r and s in place of
+ * per-mode gradients, shared reciprocals in the Roe flux, each mode loaded once per edge and
+ * the basis table in shared memory the element kernel went from 52 to 36 us, the edge kernel
+ * from 48 to 43 and a step from 267 to 197 us (163k triangles, SSP(3,3)).
  */
 #pragma once
 
@@ -26,11 +33,12 @@
 namespace dgr {
 
 /* Minimum resident blocks per SM requested for the p = 2 kernels (register caps 65536 /
- * (block size x blocks): 128 for the element kernel, 102 for the edge kernel at 128
- * threads).  Chosen by a measured sweep (1.3 M triangles, SSP(3,3): 14 % faster than the
- * uncapped 242 / 150 registers despite the spills); overridable at build time. */
+ * (block size x blocks): 128 for the element kernel, 168 for the edge kernel at 128
+ * threads), chosen by a measured sweep (163k triangles, SSP(3,3), us per step: edge kernel
+ * 196.6 with three blocks, 199.0 with four, 227.9 with five; element kernel 225.4 with four,
+ * 224.0 with three, 232.6 with five); overridable at build time. */
 #ifndef DGR_P2_MINB_EDGE
-#define DGR_P2_MINB_EDGE 5
+#define DGR_P2_MINB_EDGE 3
 #endif
 #ifndef DGR_P2_MINB_ELEMENT
 #define DGR_P2_MINB_ELEMENT 4
@@ -54,6 +62,7 @@ struct P2Ref {
     double phie[3][P2_NGP][P2_NM]; /* basis at the Gauss points of local edge k, running from
                                       vertex k to vertex k+1 */
     double mass[P2_NM];            /* int_ref phi_m^2 dr ds */
+    double imass[P2_NM];           /* 1 / mass */
 };
 
 /* per-element geometry planes of the p = 2 step */
@@ -78,45 +87,87 @@ DGR_HD int p2_match_point(int info, int g) { return (info & 128) ? g : P2_NGP - 
 
 /* ------------------------------------------------------------------ edges ---- */
 
-/* Roe flux at the 3 Gauss points of one edge, Fhat.n for the "in" element's outward normal
- * at its own Gauss points; returns the max wave speed.  Sx = the second lane of the state
- * (tangents / perturbed values) for the two-lane arithmetics, unused for T = double. */
-template <class T, class Load>
-DGR_HD T p2_edge_core(const P2Ref &ref, const Load &st, int el_in, int el_ex, int info, double nx, double ny,
-                      const T &za, const T &zb, double bz, double bq, double g, T fh[P2_NGP][3], int &code,
+/* The Roe flux of doubles with plain divisions, out of line: where the shared reciprocals
+ * (RcpDiv) are not valid. */
+static __device__ __noinline__ double p2_roe_plain(double *fh, double zeta_in, double zeta_ex, double qx_in, double qx_ex,
+                                                   double qy_in, double qy_ex, double z, double nx, double ny, double g)
+{
+    double f[3];
+    const double l = roe_flux<double>(f, zeta_in, zeta_ex, qx_in, qx_ex, qy_in, qy_ex, z, nx, ny, g, g);
+    fh[0] = f[0];
+    fh[1] = f[1];
+    fh[2] = f[2];
+    return l;
+}
+
+/* Numerical flux of one Gauss point.  Doubles on the device take the Roe flux's divisions
+ * through shared reciprocals (the same bits). */
+template <class T>
+DGR_HD T p2_flux(int ftype, T fh[3], const T ui[3], const T ue[3], const T &z, double nx, double ny, double g)
+{
+#ifdef __CUDA_ARCH__
+    if constexpr (std::is_same<T, double>::value) {
+        if (ftype == 0) {
+            RcpDiv dv;
+            double l = roe_flux_div<double>(dv, fh, ui[0], ue[0], ui[1], ue[1], ui[2], ue[2], z, nx, ny, g, g);
+            if (!dv.ok) {
+                double f[3];
+                l = p2_roe_plain(f, ui[0], ue[0], ui[1], ue[1], ui[2], ue[2], z, nx, ny, g);
+                fh[0] = f[0];
+                fh[1] = f[1];
+                fh[2] = f[2];
+            }
+            return l;
+        }
+    }
+#endif
+    return numerical_flux<T>(ftype, fh, ui[0], ue[0], ui[1], ue[1], ui[2], ue[2], z, nx, ny, g, g);
+}
+
+/* Fluxes at the 3 Gauss points of one edge, Fhat.n for the "in" element's outward normal
+ * at its own Gauss points, handed to out(gp, fh) point by point; returns the max wave speed.
+ * phie(k, gp, m): the basis at the Gauss points (mode 0 is 1); st(plane, el): the state. */
+template <class T, class Phi, class Load, class Out>
+DGR_HD T p2_edge_core(const P2Ref &ref, const Phi &phie, const Load &st, int el_in, int el_ex, int info, double nx,
+                      double ny, const T &za, const T &zb, double bz, double bq, double g, const Out &out, int &code,
                       int ftype = 0)
 {
     const int k_in = info & 3, k_ex = (info >> 2) & 3, bd = (info >> 4) & 7;
     const bool boundary = bd || el_in == el_ex;
     T lam = 0.0;
     code = 0;
+    /* the traces of each side at its three points, every mode loaded once; the ex side in
+     * the edge's order of points (p2_match_point) */
+    T ti[P2_NGP][3], tx[P2_NGP][3];
+    const auto traces = [&](int k, int el, bool turned, T u[P2_NGP][3]) {
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+            T c[P2_NM];
+#pragma unroll
+            for (int m = 0; m < P2_NM; ++m) c[m] = st(P2_NM * v + m, el);
+#pragma unroll
+            for (int gp = 0; gp < P2_NGP; ++gp) {
+                const int p = turned ? P2_NGP - 1 - gp : gp;
+                T a = c[0];
+#pragma unroll
+                for (int m = 1; m < P2_NM; ++m) a = muladd(phie(k, p, m), c[m], a);
+                u[gp][v] = a;
+            }
+        }
+    };
+    traces(k_in, el_in, false, ti);
+    if (!boundary) traces(k_ex, el_ex, !(info & 128), tx);
 #pragma unroll
     for (int gp = 0; gp < P2_NGP; ++gp) {
         const double t = ref.te[gp];
-        const T z_g = za * ((1.0 - t) / 2) + zb * ((1.0 + t) / 2);
-        T ui[3];
-#pragma unroll
-        for (int v = 0; v < 3; ++v) {
-            T a = 0.0;
-#pragma unroll
-            for (int m = 0; m < P2_NM; ++m) a += ref.phie[k_in][gp][m] * st(P2_NM * v + m, el_in);
-            ui[v] = a;
-        }
-        T ue[3];
-        if (boundary) {
-            ghost_state<T>(bd, nx, ny, ui[0], ui[1], ui[2], bz, bq, ui[0], ue[0], ue[1], ue[2]);
-        } else {
-            const int ge = p2_match_point(info, gp);
-#pragma unroll
-            for (int v = 0; v < 3; ++v) {
-                T a = 0.0;
-#pragma unroll
-                for (int m = 0; m < P2_NM; ++m) a += ref.phie[k_ex][ge][m] * st(P2_NM * v + m, el_ex);
-                ue[v] = a;
-            }
-        }
-        const T l = numerical_flux<T>(ftype, fh[gp], ui[0], ue[0], ui[1], ue[1], ui[2], ue[2], z_g, nx, ny, g, g);
-        if (isnan(fh[gp][0]) || isnan(fh[gp][1]) || isnan(fh[gp][2])) code = 1;
+        const T z_g = muladd(zb, (1.0 + t) / 2, za * ((1.0 - t) / 2));
+        if (boundary)
+            ghost_state<T>(bd, nx, ny, ti[gp][0], ti[gp][1], ti[gp][2], bz, bq, ti[gp][0], tx[gp][0], tx[gp][1],
+                           tx[gp][2]);
+        T fh[3];
+        const T l = p2_flux<T>(ftype, fh, ti[gp], tx[gp], z_g, nx, ny, g);
+        if (isnan(fh[0]) || isnan(fh[1]) || isnan(fh[2])) code = 1;
+        out(gp, fh);
         lam = rmax(lam, l);
     }
     return lam;
@@ -139,59 +190,69 @@ DGR_HD void p2_element_core(const P2Ref &ref, const T S[3][P2_NM], const T F[3][
     const T zv[3] = {zg.zv(0), zg.zv(1), zg.zv(2)};
     const T dzx = zg.dzx(), dzy = zg.dzy(), gnn = zg.gnn();
     T acc[3][P2_NM];
-#pragma unroll
-    for (int v = 0; v < 3; ++v)
-#pragma unroll
-        for (int m = 0; m < P2_NM; ++m) acc[v][m] = 0.0;
-
-    /* area integrals; the point loop stays a loop (its mode and variable indices are still
-     * compile-time): unrolled, seven copies of its body overflow the instruction cache
-     * (measured: 8 % off the p = 2 step rolled) */
-#pragma unroll 1
-    for (int q = 0; q < P2_NQ; ++q) {
-        T uq[3];
-#pragma unroll
-        for (int v = 0; v < 3; ++v) {
-            T a = 0.0;
-#pragma unroll
-            for (int m = 0; m < P2_NM; ++m) a += ref.phi[q][m] * S[v][m];
-            uq[v] = a;
-        }
-        const T zq = ref.lam[q][0] * zv[0] + ref.lam[q][1] * zv[1] + ref.lam[q][2] * zv[2];
-        const T H = uq[0] + zq;
-        const T u = uq[1] / H, vv = uq[2] / H;
-        const T p = 0.5 * g * (H * H - zq * zq);
-        const T qxy = uq[1] * vv;
-        const T fx[3] = {uq[1], uq[1] * u + p, qxy};
-        const T fy[3] = {uq[2], qxy, uq[2] * vv + p};
-        const T tau = gnn * sqrt(u * u + vv * vv) / pow43(H);
-        const T src[3] = {T(rain), g * uq[0] * dzx - tau * uq[1], g * uq[0] * dzy - tau * uq[2]};
-        const double wj = 2.0 * ref.wq[q] * detJ;
-#pragma unroll
-        for (int m = 0; m < P2_NM; ++m) {
-            const double gx = ref.dr[q][m] * rx + ref.ds[q][m] * sx;
-            const double gy = ref.dr[q][m] * ry + ref.ds[q][m] * sy;
-#pragma unroll
-            for (int v = 0; v < 3; ++v) acc[v][m] += wj * (fx[v] * gx + fy[v] * gy + src[v] * ref.phi[q][m]);
-        }
-    }
-    /* edge integrals */
+    /* edge integrals (mode 0 is 1 everywhere); first, so that the fluxes are done with */
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const double half = geo(P2G_LEN + k) / 2;
 #pragma unroll
         for (int gp = 0; gp < P2_NGP; ++gp) {
-            const double wl = ref.wg[gp] * half;
+            const double wl = -(ref.wg[gp] * half);
 #pragma unroll
-            for (int m = 0; m < P2_NM; ++m)
+            for (int v = 0; v < 3; ++v) {
+                const T f = wl * F[k][gp][v];
+                const bool first = k == 0 && gp == 0;
+                acc[v][0] = first ? f : acc[v][0] + f;
 #pragma unroll
-                for (int v = 0; v < 3; ++v) acc[v][m] -= wl * (F[k][gp][v] * ref.phie[k][gp][m]);
+                for (int m = 1; m < P2_NM; ++m)
+                    acc[v][m] = first ? ref.phie[k][gp][m] * f : muladd(ref.phie[k][gp][m], f, acc[v][m]);
+            }
         }
     }
+
+    /* area integrals; the point loop stays a loop (its mode and variable indices are still
+     * compile-time): unrolled, seven copies of its body overflow the instruction cache
+     * (measured: 8 % off the p = 2 step rolled).  F.grad phi is taken as the flux's
+     * components along r and s times the reference derivatives, which vanish for d/dr of
+     * modes 0, 1 and 3 and d/ds of mode 0. */
+#pragma unroll 1
+    for (int q = 0; q < P2_NQ; ++q) {
+        T uq[3];
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+            uq[v] = S[v][0];
+#pragma unroll
+            for (int m = 1; m < P2_NM; ++m) uq[v] = muladd(ref.phi[q][m], S[v][m], uq[v]);
+        }
+        const T zq = muladd(ref.lam[q][2], zv[2], muladd(ref.lam[q][1], zv[1], ref.lam[q][0] * zv[0]));
+        const T H = uq[0] + zq;
+        T u, vv;
+        quotient_pair(uq[1], uq[2], H, u, vv);
+        const T p = 0.5 * g * uq[0] * (H + zq); /* g (H^2 - zq^2) / 2 */
+        const T qxy = uq[1] * vv;
+        const T fx[3] = {uq[1], muladd(uq[1], u, p), qxy};
+        const T fy[3] = {uq[2], qxy, muladd(uq[2], vv, p)};
+        const T tau = gnn * sqrt(muladd(u, u, vv * vv)) / pow43(H);
+        const T gz = g * uq[0];
+        const double wj = 2.0 * ref.wq[q] * detJ;
+        const T src[3] = {T(wj * rain), wj * muladd(gz, dzx, -(tau * uq[1])), wj * muladd(gz, dzy, -(tau * uq[2]))};
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+            const T fr = wj * muladd(fy[v], ry, fx[v] * rx), fs = wj * muladd(fy[v], sy, fx[v] * sx);
+            acc[v][0] += src[v];
+#pragma unroll
+            for (int m = 1; m < P2_NM; ++m) {
+                T a = muladd(ref.phi[q][m], src[v], acc[v][m]);
+                a = muladd(ref.ds[q][m], fs, a);
+                if (m == 2 || m > 3) a = muladd(ref.dr[q][m], fr, a);
+                acc[v][m] = a;
+            }
+        }
+    }
+    const double idet = 1.0 / detJ;
     T rhs[3][P2_NM];
 #pragma unroll
     for (int m = 0; m < P2_NM; ++m) {
-        const double minv = 1.0 / (detJ * ref.mass[m]);
+        const double minv = idet * ref.imass[m];
 #pragma unroll
         for (int v = 0; v < 3; ++v) rhs[v][m] = acc[v][m] * minv;
     }
@@ -207,13 +268,13 @@ DGR_HD void p2_element_core(const P2Ref &ref, const T S[3][P2_NM], const T F[3][
 #pragma unroll
         for (int m = 0; m < P2_NM; ++m) {
             if (MODE == MODE_STAGE1) {
-                w[v][m] = S[v][m] + rhs[v][m] * dt;
+                w[v][m] = muladd(rhs[v][m], dt, S[v][m]);
             } else if (MODE == MODE_STAGE2) {
-                w[v][m] = (S[v][m] + uin(v, m)) * 0.5 + rhs[v][m] * (dt / 2);
+                w[v][m] = muladd(rhs[v][m], dt / 2, (S[v][m] + uin(v, m)) * 0.5);
             } else {
                 const double a = MODE == MODE_RK3_2 ? 0.75 : 1.0 / 3;
                 const double b = MODE == MODE_RK3_2 ? 0.25 : 2.0 / 3;
-                w[v][m] = a * uin(v, m) + b * (S[v][m] + rhs[v][m] * dt);
+                w[v][m] = muladd(b, muladd(rhs[v][m], dt, S[v][m]), a * uin(v, m));
             }
         }
 }
@@ -230,13 +291,26 @@ struct P2PlaneZ {
 
 /* --------------------------------------------------------------- kernels ---- */
 
+/* ref.phie to a block's shared memory */
+DGR_DEV void p2_load_phie(const P2Ref &ref, double *tab)
+{
+    const double *src = &ref.phie[0][0][0];
+    for (int j = threadIdx.x; j < 3 * P2_NGP * P2_NM; j += blockDim.x) tab[j] = src[j];
+    __syncthreads();
+}
+
 /* FT: the numerical flux as a compile-time constant, or -1 to take it from the mesh */
 template <int BS, int FT = -1>
-__global__ void __launch_bounds__(BS, DGR_P2_MINB_EDGE) k_p2_edge(P2Ref ref, MeshDev m, const double *__restrict__ p2g,
+__global__ void __launch_bounds__(BS, DGR_P2_MINB_EDGE) k_p2_edge(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *__restrict__ p2g,
                                                 const double *__restrict__ S, const double *__restrict__ bzeta,
                                                 const double *__restrict__ bqn, double *__restrict__ flux,
                                                 DevClock *clk, int lam_slot, int phase, double g)
 {
+    /* the local edges differ from lane to lane: the basis table in shared memory, where the
+     * few addresses of a warp meet in one or two passes instead of one each in the constant
+     * cache */
+    __shared__ double tab[3 * P2_NGP * P2_NM];
+    p2_load_phie(ref, tab);
     const int i = blockIdx.x * BS + threadIdx.x;
     const bool valid = i < m.nf;
     const int sid = (valid && m.ed_sid) ? m.ed_sid[i] : 0;
@@ -254,15 +328,16 @@ __global__ void __launch_bounds__(BS, DGR_P2_MINB_EDGE) k_p2_edge(P2Ref ref, Mes
             const double za = p2g[(size_t)(P2G_ZV + k_in) * ld + el_in];
             const double zb = p2g[(size_t)(P2G_ZV + (k_in + 1) % 3) * ld + el_in];
             const auto st = [S, ld](int plane, int el) { return S[plane * ld + el]; };
-            double fh[P2_NGP][3];
             int code;
-            lam = p2_edge_core<double>(ref, st, el_in, el_ex, info, nx, ny, za, zb, bd ? bzeta[i] : 0.0,
-                                       bd ? bqn[i] : 0.0, g, fh, code, FT >= 0 ? FT : m.flux);
+            const int lf = m.ldF;
+            const auto out = [flux, lf, i](int gp, const double fh[3]) {
+#pragma unroll
+                for (int v = 0; v < 3; ++v) flux[(3 * gp + v) * lf + i] = fh[v];
+            };
+            const auto phie = [](int k, int gp, int mm) { return tab[(k * P2_NGP + gp) * P2_NM + mm]; };
+            lam = p2_edge_core<double>(ref, phie, st, el_in, el_ex, info, nx, ny, za, zb, bd ? bzeta[i] : 0.0,
+                                       bd ? bqn[i] : 0.0, g, out, code, FT >= 0 ? FT : m.flux);
             if (code) atomicMin(&ck->err, err_key(ck->step, phase, code, i - ck->ed_off));
-#pragma unroll
-            for (int gp = 0; gp < P2_NGP; ++gp)
-#pragma unroll
-                for (int v = 0; v < 3; ++v) flux[(3 * gp + v) * m.ldF + i] = fh[gp][v];
             if (!(lam >= 0.0)) lam = 0.0;
         }
     }
@@ -292,7 +367,7 @@ DGR_HD void p2_gather_flux(const MeshDev &m, int el, const FluxLoad &fl, T F[3][
 }
 
 template <int MODE, int BS>
-__global__ void __launch_bounds__(BS, DGR_P2_MINB_ELEMENT) k_p2_element(P2Ref ref, MeshDev m, const double *__restrict__ p2g,
+__global__ void __launch_bounds__(BS, DGR_P2_MINB_ELEMENT) k_p2_element(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *__restrict__ p2g,
                                                    const double *__restrict__ S, const double *__restrict__ U,
                                                    const double *__restrict__ flux, double *__restrict__ out,
                                                    const DevClock *clk, double g)

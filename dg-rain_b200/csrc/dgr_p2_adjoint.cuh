@@ -81,18 +81,18 @@ __global__ void __launch_bounds__(128) k_p2_tlm_edge(P2Ref ref, MeshDev m, const
     const T za = lane(tag, p2g[(size_t)(P2G_ZV + k_in) * ld + el_in], zx[va]);
     const T zb = lane(tag, p2g[(size_t)(P2G_ZV + (k_in + 1) % 3) * ld + el_in], zx[vb]);
     const auto st = [S, Sx, ld, tag](int plane, int el) { return lane(tag, S[plane * ld + el], Sx[plane * ld + el]); };
-    T fh[P2_NGP][3];
     int code;
-    p2_edge_core<T>(ref, st, el_in, el_ex, info, nx, ny, za, zb, bd ? bzeta[i] : 0.0, bd ? bqn[i] : 0.0, g, fh, code,
-                    m.flux);
     const int lf = m.ldF;
-#pragma unroll
-    for (int gp = 0; gp < P2_NGP; ++gp)
+    const auto out = [flux, flux_x, lf, i](int gp, const T fh[3]) {
 #pragma unroll
         for (int v = 0; v < 3; ++v) {
-            flux[(3 * gp + v) * lf + i] = val(fh[gp][v]);
-            flux_x[(3 * gp + v) * lf + i] = second(fh[gp][v]);
+            flux[(3 * gp + v) * lf + i] = val(fh[v]);
+            flux_x[(3 * gp + v) * lf + i] = second(fh[v]);
         }
+    };
+    const auto phie = [&ref](int k, int gp, int mm) { return ref.phie[k][gp][mm]; };
+    p2_edge_core<T>(ref, phie, st, el_in, el_ex, info, nx, ny, za, zb, bd ? bzeta[i] : 0.0, bd ? bqn[i] : 0.0, g, out,
+                    code, m.flux);
 }
 
 template <int MODE, class T>
