@@ -160,34 +160,35 @@ DGR_HD void p2_area_rev(const P2Ref &ref, const double S[3][P2_NM], const double
         double uq[3];
 #pragma unroll
         for (int v = 0; v < 3; ++v) {
-            double a = 0.0;
+            uq[v] = S[v][0];
 #pragma unroll
-            for (int m = 0; m < P2_NM; ++m) a += ref.phi[q][m] * S[v][m];
-            uq[v] = a;
+            for (int m = 1; m < P2_NM; ++m) uq[v] = fma(ref.phi[q][m], S[v][m], uq[v]);
         }
-        const double zq = ref.lam[q][0] * zv[0] + ref.lam[q][1] * zv[1] + ref.lam[q][2] * zv[2];
+        const double zq = fma(ref.lam[q][2], zv[2], fma(ref.lam[q][1], zv[1], ref.lam[q][0] * zv[0]));
         const double H = uq[0] + zq;
         /* these quotients only scale derivatives (no decision depends on them): products
          * with one reciprocal per divisor, whose last bit does not matter */
         const double iH = 1.0 / H;
         const double u = uq[1] * iH, vv = uq[2] * iH;
-        const double sp = sqrt(u * u + vv * vv);
+        const double sp = sqrt(fma(u, u, vv * vv));
         const double iP = 1.0 / pow43(H);
         const double tau = gnn * sp * iP;
         const double wj = 2.0 * ref.wq[q] * detJ;
-        /* adjoints of fx, fy, src */
-        double fxb[3] = {0, 0, 0}, fyb[3] = {0, 0, 0}, srcb[3] = {0, 0, 0};
+        /* adjoints of the flux's components along r and s and of the source, then of fx, fy */
+        double fxb[3], fyb[3], srcb[3];
 #pragma unroll
-        for (int m = 0; m < P2_NM; ++m) {
-            const double gx = ref.dr[q][m] * rx + ref.ds[q][m] * sx;
-            const double gy = ref.dr[q][m] * ry + ref.ds[q][m] * sy;
+        for (int v = 0; v < 3; ++v) {
+            double frb = ref.dr[q][2] * Xb[v][2], fsb = ref.ds[q][1] * Xb[v][1];
+            srcb[v] = Xb[v][0];
 #pragma unroll
-            for (int v = 0; v < 3; ++v) {
-                const double a = wj * Xb[v][m];
-                fxb[v] += a * gx;
-                fyb[v] += a * gy;
-                srcb[v] += a * ref.phi[q][m];
+            for (int m = 1; m < P2_NM; ++m) {
+                srcb[v] = fma(ref.phi[q][m], Xb[v][m], srcb[v]);
+                if (m > 1) fsb = fma(ref.ds[q][m], Xb[v][m], fsb);
+                if (m > 3) frb = fma(ref.dr[q][m], Xb[v][m], frb);
             }
+            srcb[v] *= wj;
+            fxb[v] = wj * fma(fsb, sx, frb * rx);
+            fyb[v] = wj * fma(fsb, sy, frb * ry);
         }
         double q1b = 0, q2b = 0, zb = 0, ub = 0, vb = 0, Hb = 0, zqb = 0;
         /* fx = (q1, q1 u + p, q1 vv), fy = (q2, q1 vv, q2 vv + p) */
@@ -232,7 +233,8 @@ DGR_HD void p2_area_rev(const P2Ref &ref, const double S[3][P2_NM], const double
 #pragma unroll
         for (int v = 0; v < 3; ++v)
 #pragma unroll
-            for (int m = 0; m < P2_NM; ++m) Sb[v][m] += ref.phi[q][m] * uqb[v];
+            for (int m = 0; m < P2_NM; ++m)
+                Sb[v][m] = m == 0 ? Sb[v][0] + uqb[v] : fma(ref.phi[q][m], uqb[v], Sb[v][m]);
     }
 }
 
@@ -255,7 +257,7 @@ DGR_HD void p2_dz_rev(double rx, double ry, double sx, double sy, const double d
  * stage): every element reads its own columns before writing them.
  */
 template <int MODE>
-__global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_ELEMENT) k_p2_adj_element(P2Ref ref, MeshDev m, const double *__restrict__ p2g,
+__global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_ELEMENT) k_p2_adj_element(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *__restrict__ p2g,
                                                         const double *__restrict__ S, const double *lamO, double *lamS,
                                                         double *lamU, int u_accumulate, double *__restrict__ fbar,
                                                         double *__restrict__ zvb, double *__restrict__ nbar,
@@ -276,9 +278,10 @@ __global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_ELEMENT) k_p2_adj_element
     for (int v = 0; v < 3; ++v)
 #pragma unroll
         for (int k = 0; k < P2_NM; ++k) wb[v][k] = lamO[(P2_NM * v + k) * ld + el];
+    const double idet = 1.0 / detJ;
 #pragma unroll
     for (int k = 0; k < P2_NM; ++k) {
-        const double minv = 1.0 / (detJ * ref.mass[k]);
+        const double minv = idet * ref.imass[k];
 #pragma unroll
         for (int v = 0; v < 3; ++v) Xb[v][k] = (wb[v][k] * rk) * minv;
     }
@@ -295,9 +298,9 @@ __global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_ELEMENT) k_p2_adj_element
             const int gi = side ? p2_match_point(info, gp) : gp;
 #pragma unroll
             for (int v = 0; v < 3; ++v) {
-                double a = 0.0;
+                double a = Xb[v][0];
 #pragma unroll
-                for (int mm = 0; mm < P2_NM; ++mm) a += Xb[v][mm] * ref.phie[k][gp][mm];
+                for (int mm = 1; mm < P2_NM; ++mm) a = fma(Xb[v][mm], ref.phie[k][gp][mm], a);
                 const double fb = -wl * a;
                 fbar[(9 * side + 3 * gi + v) * m.ldF + e] = side ? -fb : fb;
             }
@@ -342,12 +345,14 @@ __global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_ELEMENT) k_p2_adj_element
  * end vertices (zeb).
  */
 template <int FT = -1>
-__global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_EDGE) k_p2_adj_edge(P2Ref ref, MeshDev m, const double *__restrict__ p2g,
+__global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_EDGE) k_p2_adj_edge(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *__restrict__ p2g,
                                                             const double *__restrict__ S,
                                                             const double *__restrict__ bzeta,
                                                             const double *__restrict__ bqn, double *__restrict__ fbar,
                                                             double *__restrict__ zeb, double g)
 {
+    __shared__ double tab[3 * P2_NGP * P2_NM]; /* as in k_p2_edge */
+    p2_load_phie(ref, tab);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.nf) return;
     const int el_in = m.e_in[i], el_ex = m.e_ex[i], info = m.e_info[i];
@@ -368,9 +373,10 @@ __global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_EDGE) k_p2_adj_edge(P2Ref
         double ui[3], ue[3];
 #pragma unroll
         for (int v = 0; v < 3; ++v) {
-            double a = 0.0;
+            double a = S[P2_NM * v * ld + el_in];
 #pragma unroll
-            for (int mm = 0; mm < P2_NM; ++mm) a += ref.phie[k_in][gp][mm] * S[(P2_NM * v + mm) * ld + el_in];
+            for (int mm = 1; mm < P2_NM; ++mm)
+                a = fma(tab[(k_in * P2_NGP + gp) * P2_NM + mm], S[(P2_NM * v + mm) * ld + el_in], a);
             ui[v] = a;
         }
         const int ge = p2_match_point(info, gp);
@@ -379,9 +385,10 @@ __global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_EDGE) k_p2_adj_edge(P2Ref
         } else {
 #pragma unroll
             for (int v = 0; v < 3; ++v) {
-                double a = 0.0;
+                double a = S[P2_NM * v * ld + el_ex];
 #pragma unroll
-                for (int mm = 0; mm < P2_NM; ++mm) a += ref.phie[k_ex][ge][mm] * S[(P2_NM * v + mm) * ld + el_ex];
+                for (int mm = 1; mm < P2_NM; ++mm)
+                    a = fma(tab[(k_ex * P2_NGP + ge) * P2_NM + mm], S[(P2_NM * v + mm) * ld + el_ex], a);
                 ue[v] = a;
             }
         }
@@ -408,7 +415,7 @@ __global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_EDGE) k_p2_adj_edge(P2Ref
 }
 
 /* trace adjoints (fbar after k_p2_adj_edge) of an element's three edges to its modes */
-static __global__ void __launch_bounds__(128) k_p2_adj_trace(P2Ref ref, MeshDev m, const double *__restrict__ fbar,
+static __global__ void __launch_bounds__(128) k_p2_adj_trace(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *__restrict__ fbar,
                                                              double *__restrict__ lamS)
 {
     const int el = blockIdx.x * blockDim.x + threadIdx.x;
@@ -431,7 +438,8 @@ static __global__ void __launch_bounds__(128) k_p2_adj_trace(P2Ref ref, MeshDev 
             for (int v = 0; v < 3; ++v) {
                 const double t = fbar[(9 * side + 3 * gi + v) * m.ldF + e];
 #pragma unroll
-                for (int mm = 0; mm < P2_NM; ++mm) a[v][mm] += ref.phie[k][gp][mm] * t;
+                for (int mm = 0; mm < P2_NM; ++mm)
+                    a[v][mm] = mm == 0 ? a[v][0] + t : fma(ref.phie[k][gp][mm], t, a[v][mm]);
             }
         }
     }
