@@ -693,7 +693,7 @@ DGR_HD LimitDecisions limit_core_rev(const double w[3][3], const Bnd &bnd, const
         const double midz[3] = {0.5 * (zn[0] + zn[1]), 0.5 * (zn[1] + zn[2]), 0.5 * (zn[2] + zn[0])};
         const double mh[3] = {wl[0][0] + midz[0], wl[0][1] + midz[1], wl[0][2] + midz[2]};
         const double ht[3] = {mh[0] - mh[1] + mh[2], mh[0] + mh[1] - mh[2], -mh[0] + mh[1] + mh[2]};
-        const double avg_h = (ht[0] + ht[1] + ht[2]) / 3;
+        const double avg_h = third(ht[0] + ht[1] + ht[2]);
         double htp[3] = {ht[0], ht[1], ht[2]};
         int mass = 0, imin = 0, inext = 1, irem = 2, takes_x = 0;
         double hmin = 0, hnext = 0;
@@ -882,7 +882,9 @@ DGR_HD LimitDecisions limit_core_rev(const double w[3][3], const Bnd &bnd, const
                             vxb[k] -= rfb;
                         }
                     } else if (bits & 1) {
-                        sumdiffb += rfb * sdd / (double)(bits >> 2);
+                        /* scales a derivative: the reciprocal of the count's last bit does not matter */
+                        const int div = bits >> 2;
+                        sumdiffb += rfb * sdd * (div == 1 ? 1.0 : (div == 2 ? 0.5 : 1.0 / 3));
                     }
                 }
                 vxb[0] += sumdiffb;

@@ -482,10 +482,10 @@ DGR_HD void limit_core(T w[3][3], const Bnd &bnd, const T zn[3], double h0, doub
         }
         T out[3][3];
         /* the limited values only count where every vertex is wet: elsewhere (dry land, the
-         * shoreline) nothing of the rest is computed, unless its path is recorded.  With the
+         * shoreline) nothing of the rest is computed or recorded.  With the
          * one division by 3 a pass can need (below) and the early end of the passes this took
          * a 4M coastal step, 30 % dry, from 2.457 to 2.323 ms, 200k from 167 to 163 us */
-        if (TRACE || modify) {
+        if (modify) {
 #pragma unroll
             for (int v = 0; v < 3; ++v) {
                 const T w1 = w[v][0], w2 = w[v][1], w3 = w[v][2];
@@ -497,7 +497,7 @@ DGR_HD void limit_core(T w[3][3], const Bnd &bnd, const T zn[3], double h0, doub
                     vmin[k] = bnd(v, k, 1);
                 }
                 const T avg = third(w1 + w2 + w3);
-                unsigned long long tb = 0;
+                unsigned long long tb = 0x540; /* sign fields of passes not reached: 0 */
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     if (TRACE) {
@@ -515,9 +515,9 @@ DGR_HD void limit_core(T w[3][3], const Bnd &bnd, const T zn[3], double h0, doub
                     const T sumloc = third(vx[0] + vx[1] + vx[2]);
                     T sumdiff = (sumloc - avg) * 3;
                     const int sd = sgn(sumdiff);
-                    if (!TRACE && sd == 0) break; /* nothing left to move: later passes change nothing */
+                    if (sd == 0) break; /* nothing left to move: later passes change nothing */
                     const double sdd = (double)sd;
-                    if (TRACE) tb |= (unsigned long long)(sd + 1) << (6 + 2 * ll);
+                    if (TRACE) tb += (unsigned long long)((long long)sd * (1ll << (6 + 2 * ll)));
                     const T diff[3] = {(vx[0] - avg) * sdd, (vx[1] - avg) * sdd, (vx[2] - avg) * sdd};
                     const int up[3] = {diff[0] > 0, diff[1] > 0, diff[2] > 0};
                     /* the reference divides by max(1, count of the vertices still to give way):
