@@ -223,7 +223,7 @@ extern "C" int dgr_set_bathymetry(dgr_ctx *c, const double *z)
 static void clock_begin_step(dgr_ctx *c, int n, int replay)
 {
     AdjointState *a = c->adj;
-    k_adj_clock_begin<<<1, 256, 0, c->stream>>>(c->clk, c->nscen, phys(c), c->bnd_edges, c->bnd_type,
+    launch_dep(k_adj_clock_begin, 1, 256, c->stream, c->clk, c->nscen, phys(c), c->bnd_edges, c->bnd_type,
                                                   c->nscen > 1 ? c->bnd_sid : nullptr, c->nbnd, c->bzeta, c->bqn,
                                                   a->dt_hist, a->time_hist, n, replay);
 }
@@ -291,7 +291,7 @@ extern "C" int dgr_adjoint_forward(dgr_ctx *c, const double *zeta, const double 
         }
         clock_begin_step(c, n, replay_dt);
         for (int st = 0; st < c->p.rk_stages; ++st) launch_stage(c, st, true);
-        k_misfit<<<blocks(a->ng, 128), 128, 0, s>>>(c->U, c->ldE, a->nw, a->ng, a->g_el, a->g_w, a->target + (size_t)n * a->ng,
+        launch_dep(k_misfit, blocks(a->ng, 128), 128, s, c->U, c->ldE, a->nw, a->ng, a->g_el, a->g_w, a->target + (size_t)n * a->ng,
                                   a->resid + (size_t)n * a->ng);
         c->launches += 2;
     }
@@ -353,7 +353,7 @@ static void recorded_stage(dgr_ctx *c, int j, int stage, const double *S, double
     if (c->p.order == 2) {
         launch_p2_edge(c, S, stage, 2 * stage);
 #define P2_EL(MD) \
-    k_p2_element<MD, 128><<<nb, 128, 0, s>>>(c->p2ref, m, c->p2g, S, U, c->flux, OUT, c->clk, c->p.g)
+    launch_dep(k_p2_element<MD, 128>, nb, 128, s, c->p2ref, m, c->p2g, S, U, c->flux, OUT, c->clk, c->p.g)
         if (mode == MODE_STAGE1)
             P2_EL(MODE_STAGE1);
         else if (mode == MODE_STAGE2)
@@ -371,19 +371,19 @@ static void recorded_stage(dgr_ctx *c, int j, int stage, const double *S, double
     launch_edge(c, S, wd_in, stage, 2 * stage);
     const unsigned ne64 = blocks(c->ne, 64); /* the element kernel in blocks of 64, as the plain step's default */
     if (mode == MODE_STAGE1)
-        k_element<MODE_STAGE1, 64><<<ne64, 64, 0, s>>>(m, S, U, wd_in, c->flux, R, avg, c->clk, c->p.g);
+        launch_dep(k_element<MODE_STAGE1, 64>, ne64, 64, s, m, S, U, wd_in, c->flux, R, avg, c->clk, c->p.g);
     else if (mode == MODE_STAGE2)
-        k_element<MODE_STAGE2, 64><<<ne64, 64, 0, s>>>(m, S, U, wd_in, c->flux, R, avg, c->clk, c->p.g);
+        launch_dep(k_element<MODE_STAGE2, 64>, ne64, 64, s, m, S, U, wd_in, c->flux, R, avg, c->clk, c->p.g);
     else if (mode == MODE_RK3_2)
-        k_element<MODE_RK3_2, 64><<<ne64, 64, 0, s>>>(m, S, U, wd_in, c->flux, R, avg, c->clk, c->p.g);
+        launch_dep(k_element<MODE_RK3_2, 64>, ne64, 64, s, m, S, U, wd_in, c->flux, R, avg, c->clk, c->p.g);
     else
-        k_element<MODE_RK3_3, 64><<<ne64, 64, 0, s>>>(m, S, U, wd_in, c->flux, R, avg, c->clk, c->p.g);
-    k_node_bounds<<<blocks(c->nn, DGR_NODE_BS), DGR_NODE_BS, 0, s>>>(m, avg, bnd);
+        launch_dep(k_element<MODE_RK3_3, 64>, ne64, 64, s, m, S, U, wd_in, c->flux, R, avg, c->clk, c->p.g);
+    launch_dep(k_node_bounds, blocks(c->nn, DGR_NODE_BS), DGR_NODE_BS, s, m, avg, bnd);
     if (wd)
-        k_limit_to<true><<<nb, 128, 0, s>>>(m, R, OUT, bnd, wd_in, wd_out, c->clk, c->p.H0, c->p.VELZERO,
+        launch_dep(k_limit_to<true>, nb, 128, s, m, R, OUT, bnd, wd_in, wd_out, c->clk, c->p.H0, c->p.VELZERO,
                                             2 * stage + 1);
     else
-        k_limit_to<false><<<nb, 128, 0, s>>>(m, R, OUT, bnd, wd_in, wd_out, c->clk, c->p.H0, c->p.VELZERO,
+        launch_dep(k_limit_to<false>, nb, 128, s, m, R, OUT, bnd, wd_in, wd_out, c->clk, c->p.H0, c->p.VELZERO,
                                              2 * stage + 1);
     c->launches += 4;
 }
@@ -403,7 +403,7 @@ static void reverse_stage_p2(dgr_ctx *c, int j, int n, int stage)
     const double g = c->p.g;
     const unsigned nb = blocks(c->ne, 128);
 #define P2_ADJ_EL(MD)                                                                                                  \
-    k_p2_adj_element<MD><<<nb, 128, 0, s>>>(c->p2ref, m, c->p2g, S, lamO, lamS, a->lamU, u_acc, a->fbar, a->zvb,    \
+    launch_dep(k_p2_adj_element<MD>, nb, 128, s, c->p2ref, m, c->p2g, S, lamO, lamS, a->lamU, u_acc, a->fbar, a->zvb,    \
                                             a->nbar, c->n_el, g, dt_row(c, n))
     if (mode == MODE_STAGE1)
         P2_ADJ_EL(MODE_STAGE1);
@@ -415,12 +415,12 @@ static void reverse_stage_p2(dgr_ctx *c, int j, int n, int stage)
         P2_ADJ_EL(MODE_RK3_3);
 #undef P2_ADJ_EL
     if (c->p.flux == 0)
-        k_p2_adj_edge<0><<<blocks(c->nf, 128), 128, 0, s>>>(c->p2ref, m, c->p2g, S, c->bzeta, c->bqn, a->fbar, a->zeb,
+        launch_dep(k_p2_adj_edge<0>, blocks(c->nf, 128), 128, s, c->p2ref, m, c->p2g, S, c->bzeta, c->bqn, a->fbar, a->zeb,
                                                             g);
     else
-        k_p2_adj_edge<-1><<<blocks(c->nf, 128), 128, 0, s>>>(c->p2ref, m, c->p2g, S, c->bzeta, c->bqn, a->fbar,
+        launch_dep(k_p2_adj_edge<-1>, blocks(c->nf, 128), 128, s, c->p2ref, m, c->p2g, S, c->bzeta, c->bqn, a->fbar,
                                                              a->zeb, g);
-    k_p2_adj_trace<<<nb, 128, 0, s>>>(c->p2ref, m, a->fbar, lamS);
+    launch_dep(k_p2_adj_trace, nb, 128, s, c->p2ref, m, a->fbar, lamS);
     c->launches += 3;
 }
 
@@ -447,14 +447,14 @@ static void reverse_stage(dgr_ctx *c, int j, int n, int stage)
     const double h0 = c->p.H0, vz = c->p.VELZERO, g = c->p.g;
     const unsigned nb = blocks(c->ne, 128);
     if (wd)
-        k_adj_limit<true><<<nb, 128, 0, s>>>(m, seg_R(c, j, stage), seg_B(c, j, stage), lamO, a->Rbar, a->bbar, a->zvb,
+        launch_dep(k_adj_limit<true>, nb, 128, s, m, seg_R(c, j, stage), seg_B(c, j, stage), lamO, a->Rbar, a->bbar, a->zvb,
                                              h0, vz);
     else
-        k_adj_limit<false><<<nb, 128, 0, s>>>(m, seg_R(c, j, stage), seg_B(c, j, stage), lamO, a->Rbar, a->bbar,
+        launch_dep(k_adj_limit<false>, nb, 128, s, m, seg_R(c, j, stage), seg_B(c, j, stage), lamO, a->Rbar, a->bbar,
                                               a->zvb, h0, vz);
-    k_adj_node<<<blocks(c->nn, 256), 256, 0, s>>>(m, seg_avg(c, j, stage), a->bbar, a->bnode, a->barg);
+    launch_dep(k_adj_node, blocks(c->nn, 256), 256, s, m, seg_avg(c, j, stage), a->bbar, a->bnode, a->barg);
 #define ADJ_EL(MD)                                                                                                 \
-    k_adj_element<MD><<<nb, 128, 0, s>>>(m, S, wd_in, a->Rbar, a->bnode, a->barg, lamS, a->lamU, u_acc, a->fbar,   \
+    launch_dep(k_adj_element<MD>, nb, 128, s, m, S, wd_in, a->Rbar, a->bnode, a->barg, lamS, a->lamU, u_acc, a->fbar,   \
                                          a->zvb, a->nbar, c->n_el, g, dt_row(c, n))
     if (mode == MODE_STAGE1)
         ADJ_EL(MODE_STAGE1);
@@ -466,7 +466,7 @@ static void reverse_stage(dgr_ctx *c, int j, int n, int stage)
         ADJ_EL(MODE_RK3_3);
 #undef ADJ_EL
 #define ADJ_EDGE(W, F) \
-    k_adj_edge<W, F><<<blocks(c->nf, DGR_ADJ_EDGE_BS), DGR_ADJ_EDGE_BS, 0, s>>>(m, S, wd_in, c->bzeta, c->bqn,   \
+    launch_dep(k_adj_edge<W, F>, blocks(c->nf, DGR_ADJ_EDGE_BS), DGR_ADJ_EDGE_BS, s, m, S, wd_in, c->bzeta, c->bqn,   \
                                                                           a->fbar, lamS, a->zeb, g)
     if (c->p.flux == 0) { /* the reference's Roe flux, compiled alone */
         if (wd)
@@ -549,9 +549,9 @@ extern "C" int dgr_adjoint_backward(dgr_ctx *c, double *grad_n_el, double *grad_
         /* 2. reverse the segment */
         for (int j = len - 1; j >= 0; --j) {
             const int n = n0 + j;
-            replay_forcing(c, n);
-            k_misfit_rev<<<blocks(a->nu, 128), 128, 0, s>>>(a->lamU, c->ldE, a->nw, a->nu, a->u_el, a->u_ptr, a->u_g,
-                                                            a->g_w, a->resid + (size_t)n * a->ng);
+            launch_dep(k_adj_step_rev, blocks(c->nbnd + a->nu, 256), 256, s, c->clk, a->time_hist, n, nsc, c->bnd_edges,
+                       c->bnd_type, nsc > 1 ? c->bnd_sid : nullptr, c->nbnd, c->bzeta, c->bqn, a->lamU, c->ldE, a->nw,
+                       a->nu, a->u_el, a->u_ptr, a->u_g, a->g_w, a->resid + (size_t)n * a->ng);
             c->launches++;
             for (int st = ns - 1; st >= 0; --st) reverse_stage(c, j, n, st);
         }

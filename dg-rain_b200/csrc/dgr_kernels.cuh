@@ -294,8 +294,8 @@ DGR_DEV void copy_async4(int *dst, const int *src)
  * 114 -> 111, ensemble of 32 (0.9M) 482 -> 469, 24k 58.1 -> 57.9, 1,600 45.1 -> 45.0. */
 template <bool WD, int FT, bool ENS>
 __global__ void __launch_bounds__(DGR_EDGE_BS, DGR_MINB_EDGE)
-    k_edge_flux(const __grid_constant__ MeshDev m, const double *__restrict__ S, const int *__restrict__ wd,
-                const double *__restrict__ bzeta, const double *__restrict__ bqn, double *__restrict__ flux,
+    k_edge_flux(const __grid_constant__ MeshDev m, const double *S, const int *wd,
+                const double *bzeta, const double *bqn, double *flux,
                 DevClock *clk, int lam_slot, int phase, double g)
 {
     constexpr int BS = DGR_EDGE_BS;
@@ -453,10 +453,10 @@ DGR_DEV void element_item(const MeshDev &m, const double *S, const double *U, co
 }
 
 template <int MODE, int BS>
-__global__ void __launch_bounds__(BS, DGR_ELEMENT_THREADS_PER_SM / BS) k_element(const __grid_constant__ MeshDev m, const double *__restrict__ S,
-                                                          const double *__restrict__ U, const int *__restrict__ wd,
-                                                          const double *__restrict__ flux, double *__restrict__ out,
-                                                          double *__restrict__ avg, const DevClock *clk, double g)
+__global__ void __launch_bounds__(BS, DGR_ELEMENT_THREADS_PER_SM / BS) k_element(const __grid_constant__ MeshDev m, const double *S,
+                                                          const double *U, const int *wd,
+                                                          const double *flux, double *out,
+                                                          double *avg, const DevClock *clk, double g)
 {
     /* the block's geometry planes are requested from DRAM at once instead of in the order
      * the element computation reaches them (measured: 4 % off this kernel) */
@@ -504,8 +504,8 @@ DGR_DEV void node_item(const MeshDev &m, const double *avg, double *bounds, int 
 #ifndef DGR_NODE_BS /* threads per block of the node-bounds kernel */
 #define DGR_NODE_BS 256
 #endif
-static __global__ void __launch_bounds__(DGR_NODE_BS) k_node_bounds(MeshDev m, const double *__restrict__ avg,
-                                                     double *__restrict__ bounds)
+static __global__ void __launch_bounds__(DGR_NODE_BS) k_node_bounds(MeshDev m, const double *avg,
+                                                     double *bounds)
 {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n < m.nn) node_item(m, avg, bounds, n);
@@ -583,11 +583,11 @@ DGR_DEV void limit_item(const MeshDev &m, double *S, const double *bounds, const
 }
 
 template <bool LIMIT, bool PDOP, bool STATUS, int BS>
-__global__ void __launch_bounds__(BS, DGR_LIMIT_THREADS_PER_SM / BS) k_limit(const __grid_constant__ MeshDev m, double *__restrict__ S,
-                                                        const double *__restrict__ bounds,
-                                                        const int *__restrict__ wd_in, int *__restrict__ wd_out,
+__global__ void __launch_bounds__(BS, DGR_LIMIT_THREADS_PER_SM / BS) k_limit(const __grid_constant__ MeshDev m, double *S,
+                                                        const double *bounds,
+                                                        const int *wd_in, int *wd_out,
                                                         DevClock *clk, double h0, double velzero, int phase,
-                                                        int *__restrict__ dec_limit, int *__restrict__ dec_pdop)
+                                                        int *dec_limit, int *dec_pdop)
 {
     const int el = blockIdx.x * BS + threadIdx.x;
     if (el < m.ne)
@@ -661,10 +661,10 @@ DGR_DEV void clock_begin_body(DevClock *clk, int nscen, const PhysParams &p, con
 }
 
 static __global__ void __launch_bounds__(256) k_clock_begin(DevClock *clk, int nscen, PhysParams p,
-                                                     const int *__restrict__ bnd_edges,
-                                                     const int *__restrict__ bnd_type,
-                                                     const int *__restrict__ bnd_sid, int nbnd,
-                                                     double *__restrict__ bzeta, double *__restrict__ bqn)
+                                                     const int *bnd_edges,
+                                                     const int *bnd_type,
+                                                     const int *bnd_sid, int nbnd,
+                                                     double *bzeta, double *bqn)
 {
     pdl_wait();
     pdl_trigger();
@@ -691,9 +691,9 @@ static __global__ void k_clock_finish(DevClock *clk, int nscen, PhysParams p)
  * zeta_g = sum_k w[nm g + k] zeta_k(el_g) for the step count of the gauge's scenario, the
  * step whose end is still to be taken included (a finished scenario rewrites its last row
  * with the same state). */
-static __global__ void k_gauge_record(const double *__restrict__ S, int ld, int nm, int ng, const int *__restrict__ g_el,
-                                      const int *__restrict__ g_sid, const double *__restrict__ g_w,
-                                      const DevClock *clk, int cap, double *__restrict__ series)
+static __global__ void k_gauge_record(const double *S, int ld, int nm, int ng, const int *g_el,
+                                      const int *g_sid, const double *g_w,
+                                      const DevClock *clk, int cap, double *series)
 {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ng) return;

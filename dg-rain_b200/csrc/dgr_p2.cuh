@@ -301,9 +301,9 @@ DGR_DEV void p2_load_phie(const P2Ref &ref, double *tab)
 
 /* FT: the numerical flux as a compile-time constant, or -1 to take it from the mesh */
 template <int BS, int FT = -1>
-__global__ void __launch_bounds__(BS, DGR_P2_MINB_EDGE) k_p2_edge(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *__restrict__ p2g,
-                                                const double *__restrict__ S, const double *__restrict__ bzeta,
-                                                const double *__restrict__ bqn, double *__restrict__ flux,
+__global__ void __launch_bounds__(BS, DGR_P2_MINB_EDGE) k_p2_edge(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *p2g,
+                                                const double *S, const double *bzeta,
+                                                const double *bqn, double *flux,
                                                 DevClock *clk, int lam_slot, int phase, double g)
 {
     /* the local edges differ from lane to lane: the basis table in shared memory, where the
@@ -367,9 +367,9 @@ DGR_HD void p2_gather_flux(const MeshDev &m, int el, const FluxLoad &fl, T F[3][
 }
 
 template <int MODE, int BS>
-__global__ void __launch_bounds__(BS, DGR_P2_MINB_ELEMENT) k_p2_element(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *__restrict__ p2g,
-                                                   const double *__restrict__ S, const double *__restrict__ U,
-                                                   const double *__restrict__ flux, double *__restrict__ out,
+__global__ void __launch_bounds__(BS, DGR_P2_MINB_ELEMENT) k_p2_element(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *p2g,
+                                                   const double *S, const double *U,
+                                                   const double *flux, double *out,
                                                    const DevClock *clk, double g)
 {
     const int el = blockIdx.x * BS + threadIdx.x;

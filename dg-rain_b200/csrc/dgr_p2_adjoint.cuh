@@ -257,12 +257,12 @@ DGR_HD void p2_dz_rev(double rx, double ry, double sx, double sy, const double d
  * stage): every element reads its own columns before writing them.
  */
 template <int MODE>
-__global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_ELEMENT) k_p2_adj_element(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *__restrict__ p2g,
-                                                        const double *__restrict__ S, const double *lamO, double *lamS,
-                                                        double *lamU, int u_accumulate, double *__restrict__ fbar,
-                                                        double *__restrict__ zvb, double *__restrict__ nbar,
-                                                        const double *__restrict__ n_el, double g,
-                                                        const double *__restrict__ dt_n)
+__global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_ELEMENT) k_p2_adj_element(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *p2g,
+                                                        const double *S, const double *lamO, double *lamS,
+                                                        double *lamU, int u_accumulate, double *fbar,
+                                                        double *zvb, double *nbar,
+                                                        const double *n_el, double g,
+                                                        const double *dt_n)
 {
     const int el = blockIdx.x * blockDim.x + threadIdx.x;
     if (el >= m.ne) return;
@@ -270,6 +270,8 @@ __global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_ELEMENT) k_p2_adj_element
     const double *G = p2g + el;
     const double detJ = G[0], rx = G[(size_t)P2G_RX * ld], ry = G[(size_t)P2G_RY * ld];
     const double sx = G[(size_t)P2G_SX * ld], sy = G[(size_t)P2G_SY * ld];
+    pdl_wait();
+    pdl_trigger();
     double cu, cs, cr;
     stage_coefficients(MODE, cu, cs, cr);
     const double rk = MODE == MODE_RHS ? 1.0 : cr * dt_n[m.el_sid ? m.el_sid[el] : 0];
@@ -345,11 +347,11 @@ __global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_ELEMENT) k_p2_adj_element
  * end vertices (zeb).
  */
 template <int FT = -1>
-__global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_EDGE) k_p2_adj_edge(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *__restrict__ p2g,
-                                                            const double *__restrict__ S,
-                                                            const double *__restrict__ bzeta,
-                                                            const double *__restrict__ bqn, double *__restrict__ fbar,
-                                                            double *__restrict__ zeb, double g)
+__global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_EDGE) k_p2_adj_edge(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *p2g,
+                                                            const double *S,
+                                                            const double *bzeta,
+                                                            const double *bqn, double *fbar,
+                                                            double *zeb, double g)
 {
     __shared__ double tab[3 * P2_NGP * P2_NM]; /* as in k_p2_edge */
     p2_load_phie(ref, tab);
@@ -362,6 +364,8 @@ __global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_EDGE) k_p2_adj_edge(const
     const int ld = m.ldE, lf = m.ldF;
     const double za = p2g[(size_t)(P2G_ZV + k_in) * ld + el_in];
     const double zb = p2g[(size_t)(P2G_ZV + (k_in + 1) % 3) * ld + el_in];
+    pdl_wait();
+    pdl_trigger();
     const double bz = bd ? bzeta[i] : 0.0, bq = bd ? bqn[i] : 0.0;
     double zab = 0, zbb = 0;
     /* a loop (instruction cache; nothing here is indexed by the point but the tables and
@@ -415,12 +419,14 @@ __global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_EDGE) k_p2_adj_edge(const
 }
 
 /* trace adjoints (fbar after k_p2_adj_edge) of an element's three edges to its modes */
-static __global__ void __launch_bounds__(128) k_p2_adj_trace(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *__restrict__ fbar,
-                                                             double *__restrict__ lamS)
+static __global__ void __launch_bounds__(128) k_p2_adj_trace(const __grid_constant__ P2Ref ref, const __grid_constant__ MeshDev m, const double *fbar,
+                                                             double *lamS)
 {
     const int el = blockIdx.x * blockDim.x + threadIdx.x;
     if (el >= m.ne) return;
     const int ld = m.ldE;
+    pdl_wait();
+    pdl_trigger();
     double a[3][P2_NM];
 #pragma unroll
     for (int v = 0; v < 3; ++v)

@@ -103,18 +103,20 @@ DGR_DEV void edge_vertices(const MeshDev &m, int el_in, int k_in, int &va, int &
  * recomputation; same arithmetic).  Without wet/dry the flags pass through unchanged, as
  * the plain step keeps using the same array. */
 template <bool WD>
-__global__ void __launch_bounds__(128) k_limit_to(MeshDev m, const double *__restrict__ R, double *__restrict__ S,
-                                                  const double *__restrict__ bounds, const int *__restrict__ wd_in,
-                                                  int *__restrict__ wd_out, DevClock *clk, double h0, double velzero,
+__global__ void __launch_bounds__(128) k_limit_to(MeshDev m, const double *R, double *S,
+                                                  const double *bounds, const int *wd_in,
+                                                  int *wd_out, DevClock *clk, double h0, double velzero,
                                                   int phase)
 {
     const int el = blockIdx.x * blockDim.x + threadIdx.x;
     if (el >= m.ne) return;
     DevClock *ck = clk;
-    if (ck->done) return;
     const int ld = m.ldE;
     const int nd[3] = {m.el2v[el], m.el2v[ld + el], m.el2v[2 * ld + el]};
     const double zn[3] = {m.zn[nd[0]], m.zn[nd[1]], m.zn[nd[2]]};
+    pdl_wait();
+    pdl_trigger();
+    if (ck->done) return;
     double w[3][3];
 #pragma unroll
     for (int v = 0; v < 3; ++v)
@@ -136,12 +138,14 @@ __global__ void __launch_bounds__(128) k_limit_to(MeshDev m, const double *__res
  * records each scenario's boundary-value time and dt of the step (histories [step][nscen]),
  * then clock_begin_body. */
 static __global__ void __launch_bounds__(256) k_adj_clock_begin(DevClock *clk, int nscen, PhysParams p,
-                                                         const int *__restrict__ bnd_edges,
-                                                         const int *__restrict__ bnd_type,
-                                                         const int *__restrict__ bnd_sid, int nbnd,
-                                                         double *__restrict__ bzeta, double *__restrict__ bqn,
+                                                         const int *bnd_edges,
+                                                         const int *bnd_type,
+                                                         const int *bnd_sid, int nbnd,
+                                                         double *bzeta, double *bqn,
                                                          double *dt_hist, double *time_hist, int n, int replay)
 {
+    pdl_wait();
+    pdl_trigger();
     const size_t row = (size_t)n * nscen;
     for (int s = threadIdx.x; s < nscen; s += blockDim.x) {
         clock_end_item(clk + s);
@@ -158,16 +162,11 @@ static __global__ void __launch_bounds__(256) k_adj_clock_begin(DevClock *clk, i
         for (int s = threadIdx.x; s < nscen; s += blockDim.x) dt_hist[row + s] = clk[s].dt;
 }
 
-/* boundary_conditions() at the recorded time of step n (each prescribed edge at its
+/* boundary_conditions() at the recorded time of step n for prescribed edge j (at its
  * scenario's time) */
-static __global__ void __launch_bounds__(256) k_adj_forcing(const DevClock *clk, const double *__restrict__ time_hist, int n,
-                                                     int nscen, const int *__restrict__ bnd_edges,
-                                                     const int *__restrict__ bnd_type,
-                                                     const int *__restrict__ bnd_sid, int nbnd,
-                                                     double *__restrict__ bzeta, double *__restrict__ bqn)
+DGR_DEV void replay_forcing_item(const DevClock *clk, const double *time_hist, int n, int nscen, const int *bnd_edges,
+                                 const int *bnd_type, const int *bnd_sid, int j, double *bzeta, double *bqn)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nbnd) return;
     const int sid = bnd_sid ? bnd_sid[j] : 0;
     const DevClock *ck = clk + sid;
     const double zb2 = dgr_outflow_zeta(time_hist[(size_t)n * nscen + sid], ck->tide_on, ck->tide_amp, ck->tide_period);
@@ -181,13 +180,25 @@ static __global__ void __launch_bounds__(256) k_adj_forcing(const DevClock *clk,
     bqn[e] = qn;
 }
 
+static __global__ void __launch_bounds__(256) k_adj_forcing(const DevClock *clk, const double *__restrict__ time_hist, int n,
+                                                     int nscen, const int *__restrict__ bnd_edges,
+                                                     const int *__restrict__ bnd_type,
+                                                     const int *__restrict__ bnd_sid, int nbnd,
+                                                     double *__restrict__ bzeta, double *__restrict__ bqn)
+{
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < nbnd) replay_forcing_item(clk, time_hist, n, nscen, bnd_edges, bnd_type, bnd_sid, j, bzeta, bqn);
+}
+
 /* Gauge residuals of the state after step n: r_g = sum_k w_gk zeta_k(el_g) - target_g
  * (target null: 0), nw weights per gauge over the elevation planes 0..nw-1 (the three
  * midpoint values at p = 1, the six modes at p = 2).  One thread per gauge; the objective
  * is summed later in a fixed order. */
-static __global__ void k_misfit(const double *__restrict__ S, int ld, int nw, int ng, const int *__restrict__ g_el,
-                         const double *__restrict__ g_w, const double *__restrict__ target, double *__restrict__ resid)
+static __global__ void k_misfit(const double *S, int ld, int nw, int ng, const int *g_el,
+                         const double *g_w, const double *target, double *resid)
 {
+    pdl_wait();
+    pdl_trigger();
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ng; g += gridDim.x * blockDim.x) {
         const int el = g_el[g];
         double z = g_w[nw * g] * S[el];
@@ -212,20 +223,32 @@ static __global__ void k_misfit_sum(const double *__restrict__ resid, const doub
     out[1] = J2;
 }
 
-/* adjoint of the misfit of step n: lam(zeta_k) += 2 r_g w_gk at the gauges.  One thread per
- * gauge element (u_el, CSR u_ptr/u_g of its gauges in ascending order), so gauges that share
- * an element are added in a fixed order. */
-static __global__ void k_misfit_rev(double *__restrict__ lam, int ld, int nw, int nu, const int *__restrict__ u_el,
-                                    const int *__restrict__ u_ptr, const int *__restrict__ u_g,
-                                    const double *__restrict__ g_w, const double *__restrict__ resid)
+/* Start of the reverse of step n: threads 0..nbnd-1 write the step's boundary values
+ * (replay_forcing_item), the next nu threads add the adjoint of its misfit,
+ * lam(zeta_k) += 2 r_g w_gk at the gauges.  One thread per gauge element (u_el, CSR u_ptr/u_g
+ * of its gauges in ascending order), so gauges that share an element are added in a fixed
+ * order. */
+static __global__ void __launch_bounds__(256) k_adj_step_rev(
+    const DevClock *clk, const double *time_hist, int n, int nscen, const int *bnd_edges,
+    const int *bnd_type, const int *bnd_sid, int nbnd, double *bzeta,
+    double *bqn, double *lam, int ld, int nw, int nu, const int *u_el,
+    const int *u_ptr, const int *u_g, const double *g_w,
+    const double *resid)
 {
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < nbnd) {
+        replay_forcing_item(clk, time_hist, n, nscen, bnd_edges, bnd_type, bnd_sid, j, bzeta, bqn);
+        return;
+    }
+    const int u = j - nbnd;
     if (u >= nu) return;
     const int el = u_el[u];
     for (int k = 0; k < nw; ++k) {
         double a = lam[(size_t)k * ld + el];
-        for (int j = u_ptr[u]; j < u_ptr[u + 1]; ++j) {
-            const int g = u_g[j];
+        for (int i = u_ptr[u]; i < u_ptr[u + 1]; ++i) {
+            const int g = u_g[i];
             a += 2.0 * resid[g] * g_w[nw * g + k];
         }
         lam[(size_t)k * ld + el] = a;
@@ -414,10 +437,10 @@ __global__ void __launch_bounds__(128) k_tlm_limit(MeshDev m, double *__restrict
 
 /* limiter + PDop reverse of one element */
 template <bool WD>
-__global__ void __launch_bounds__(128, DGR_ADJ_MINB_LIMIT) k_adj_limit(MeshDev m, const double *__restrict__ R,
-                                                   const double *__restrict__ bounds,
-                                                   const double *__restrict__ lamO, double *__restrict__ Rbar,
-                                                   double *__restrict__ bbar, double *__restrict__ zvb, double h0,
+__global__ void __launch_bounds__(128, DGR_ADJ_MINB_LIMIT) k_adj_limit(MeshDev m, const double *R,
+                                                   const double *bounds,
+                                                   const double *lamO, double *Rbar,
+                                                   double *bbar, double *zvb, double h0,
                                                    double velzero)
 {
     const int el = blockIdx.x * blockDim.x + threadIdx.x;
@@ -425,6 +448,8 @@ __global__ void __launch_bounds__(128, DGR_ADJ_MINB_LIMIT) k_adj_limit(MeshDev m
     const int ld = m.ldE;
     const int nd[3] = {m.el2v[el], m.el2v[ld + el], m.el2v[2 * ld + el]};
     const double zn[3] = {m.zn[nd[0]], m.zn[nd[1]], m.zn[nd[2]]};
+    pdl_wait();
+    pdl_trigger();
     double w[3][3], wb[3][3];
 #pragma unroll
     for (int v = 0; v < 3; ++v)
@@ -452,9 +477,9 @@ __global__ void __launch_bounds__(128, DGR_ADJ_MINB_LIMIT) k_adj_limit(MeshDev m
 
 /* node bounds reverse: which element supplied each max/min, and the bound adjoints summed
  * over the elements around the node (in the node's element order) */
-static __global__ void __launch_bounds__(256) k_adj_node(MeshDev m, const double *__restrict__ avg,
-                                                  const double *__restrict__ bbar, double *__restrict__ bnode,
-                                                  int *__restrict__ barg)
+static __global__ void __launch_bounds__(256) k_adj_node(MeshDev m, const double *avg,
+                                                  const double *bbar, double *bnode,
+                                                  int *barg)
 {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= m.nn) return;
@@ -462,7 +487,10 @@ static __global__ void __launch_bounds__(256) k_adj_node(MeshDev m, const double
     double mx[3] = {-99999, -99999, -99999}, mn[3] = {99999, 99999, 99999};
     int imx[3] = {-1, -1, -1}, imn[3] = {-1, -1, -1};
     double s[6] = {0, 0, 0, 0, 0, 0};
-    for (int j = m.n2e_ptr[n]; j < m.n2e_ptr[n + 1]; ++j) {
+    const int first = m.n2e_ptr[n], last = m.n2e_ptr[n + 1];
+    pdl_wait();
+    pdl_trigger();
+    for (int j = first; j < last; ++j) {
         const int el = m.n2e[j];
 #pragma unroll
         for (int v = 0; v < 3; ++v) {
@@ -495,26 +523,27 @@ static __global__ void __launch_bounds__(256) k_adj_node(MeshDev m, const double
  * stage of RK3 (u_accumulate = 1).  Also writes the per-edge-side flux adjoints and
  * accumulates the depth / Manning adjoints. */
 template <int MODE>
-__global__ void __launch_bounds__(128, DGR_ADJ_MINB_ELEMENT) k_adj_element(MeshDev m, const double *__restrict__ S,
-                                                     const int *__restrict__ wd, const double *__restrict__ Rbar,
-                                                     const double *__restrict__ bnode, const int *__restrict__ barg,
+__global__ void __launch_bounds__(128, DGR_ADJ_MINB_ELEMENT) k_adj_element(MeshDev m, const double *S,
+                                                     const int *wd, const double *Rbar,
+                                                     const double *bnode, const int *barg,
                                                      double *lamS, double *lamU, int u_accumulate,
-                                                     double *__restrict__ fbar, double *__restrict__ zvb,
-                                                     double *__restrict__ nbar, const double *__restrict__ n_el,
-                                                     double g, const double *__restrict__ dt_n)
+                                                     double *fbar, double *zvb,
+                                                     double *nbar, const double *n_el,
+                                                     double g, const double *dt_n)
 {
     prefetch_geometry(m, blockIdx.x * blockDim.x, min((int)blockDim.x, m.ne - (int)(blockIdx.x * blockDim.x)));
     const int el = blockIdx.x * blockDim.x + threadIdx.x;
     if (el >= m.ne) return;
     const int ld = m.ldE, lb = m.ldN;
+    const int nd[3] = {m.el2v[el], m.el2v[ld + el], m.el2v[2 * ld + el]};
+    pdl_wait();
+    pdl_trigger();
     double ab[3] = {0, 0, 0};
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const int nd = m.el2v[k * ld + el];
+    for (int k = 0; k < 3; ++k)
 #pragma unroll
         for (int q = 0; q < 6; ++q)
-            if (barg[q * lb + nd] == el) ab[q % 3] += bnode[q * lb + nd];
-    }
+            if (barg[q * lb + nd[k]] == el) ab[q % 3] += bnode[q * lb + nd[k]];
     double wb[3][3];
 #pragma unroll
     for (int v = 0; v < 3; ++v)
@@ -566,16 +595,18 @@ __global__ void __launch_bounds__(128, DGR_ADJ_MINB_ELEMENT) k_adj_element(MeshD
 /* edge reverse: Roe flux(es), ghost states; adds the trace adjoints into the slots of the
  * adjacent elements (each slot belongs to one edge side) and the mid-edge depth adjoint */
 template <bool WD, int FT = -1>
-__global__ void __launch_bounds__(DGR_ADJ_EDGE_BS, DGR_ADJ_MINB_EDGE) k_adj_edge(MeshDev m, const double *__restrict__ S, const int *__restrict__ wd,
-                                                  const double *__restrict__ bzeta, const double *__restrict__ bqn,
-                                                  const double *__restrict__ fbar, double *__restrict__ lamS,
-                                                  double *__restrict__ zeb, double g)
+__global__ void __launch_bounds__(DGR_ADJ_EDGE_BS, DGR_ADJ_MINB_EDGE) k_adj_edge(MeshDev m, const double *S, const int *wd,
+                                                  const double *bzeta, const double *bqn,
+                                                  const double *fbar, double *lamS,
+                                                  double *zeb, double g)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.nf) return;
     const int el_in = m.e_in[i], el_ex = m.e_ex[i], info = m.e_info[i];
     const int k_in = info & 3, k_ex = (info >> 2) & 3, bd = (info >> 4) & 7;
     const double nx = m.e_geo[i], ny = m.e_geo[m.ldF + i], z_edge = m.e_geo[2 * m.ldF + i];
+    pdl_wait();
+    pdl_trigger();
     const int ld = m.ldE;
     const double zi = S[k_in * ld + el_in], qxi = S[(3 + k_in) * ld + el_in], qyi = S[(6 + k_in) * ld + el_in];
     const bool boundary = bd || el_in == el_ex;
