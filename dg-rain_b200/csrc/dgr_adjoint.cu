@@ -368,9 +368,12 @@ static void recorded_stage(dgr_ctx *c, int j, int stage, const double *S, double
     }
     const bool wd = c->p.wet_dry != 0;
     double *R = seg_R(c, j, stage), *avg = seg_avg(c, j, stage), *bnd = seg_B(c, j, stage);
-    launch_edge(c, S, wd_in, stage, 2 * stage);
     const unsigned ne64 = blocks(c->ne, 64); /* the element kernel in blocks of 64, as the plain step's default */
-    if (mode == MODE_STAGE1)
+    const bool together = edges_with_elements(c);
+    if (!together) launch_edge(c, S, wd_in, stage, 2 * stage);
+    if (together)
+        launch_edge_element(c, mode, S, U, wd_in, R, avg, stage);
+    else if (mode == MODE_STAGE1)
         launch_dep(k_element<MODE_STAGE1, 64>, ne64, 64, s, m, S, U, wd_in, c->flux, R, avg, c->clk, c->p.g);
     else if (mode == MODE_STAGE2)
         launch_dep(k_element<MODE_STAGE2, 64>, ne64, 64, s, m, S, U, wd_in, c->flux, R, avg, c->clk, c->p.g);
@@ -385,7 +388,7 @@ static void recorded_stage(dgr_ctx *c, int j, int stage, const double *S, double
     else
         launch_dep(k_limit_to<false>, nb, 128, s, m, R, OUT, bnd, wd_in, wd_out, c->clk, c->p.H0, c->p.VELZERO,
                                              2 * stage + 1);
-    c->launches += 4;
+    c->launches += together ? 3 : 4;
 }
 
 /* reverse of one p = 2 stage: element, edge, trace gather */

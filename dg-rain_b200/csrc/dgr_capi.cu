@@ -214,6 +214,21 @@ static int upload_concat(cudaStream_t s, T *dst, int nscen, const T *const *src,
     return DGR_OK;
 }
 
+/* Largest mesh (elements) whose edges and elements share a launch (Roe flux), and whose limiter
+ * takes the node bounds itself: where a launch costs more than the work it saves from being done
+ * twice.  us per step with a launch of each kind, with the limiter's fold, with both: 1,600
+ * triangles 44.6, 42.7, 36.8; 8,000 48.7, 46.0, 45.0; 16,000 52.5, 49.6, 50.3; 24k 57.3, 53.7,
+ * 62.7; 50,000 68.5, 64.9, 77.4; RK3 HLLC 6,000 51.1, 44.5, 45.5 and 91k 113.4, 110.1, 124.7;
+ * 200k 165.7, 170.0, 246. */
+#ifndef DGR_EDGE_ELEMENT_MAX
+#define DGR_EDGE_ELEMENT_MAX 8000
+#endif
+#ifndef DGR_FOLD_LIMIT_MAX
+#define DGR_FOLD_LIMIT_MAX 100000
+#endif
+bool edges_with_elements(const dgr_ctx *c) { return c->ne <= DGR_EDGE_ELEMENT_MAX && c->p.flux == 0; }
+static bool limiter_folds_nodes(const dgr_ctx *c) { return c->ne <= DGR_FOLD_LIMIT_MAX; }
+
 /* One shared-memory carveout for the p = 1 step's kernels: what four resident blocks of
  * k_edge_flux need.  An SM changes its carveout only when it is empty, so with the driver's
  * choice per kernel (least for the others) no block of the next kernel starts while the edge
@@ -232,6 +247,17 @@ static void set_carveouts(const dgr_ctx *c)
             set(k_edge_flux<decltype(wd)::value, decltype(ft)::value, false>);
     };
     const auto edges = [&](auto wd) {
+        constexpr bool W = decltype(wd)::value;
+        if (limiter_folds_nodes(c)) set(k_fold_limit<true, W, W>);
+        if (edges_with_elements(c)) {
+            set(k_edge_element<MODE_STAGE1, W>);
+            if (c->p.rk_stages == 3) {
+                set(k_edge_element<MODE_RK3_2, W>);
+                set(k_edge_element<MODE_RK3_3, W>);
+            } else {
+                set(k_edge_element<MODE_STAGE2, W>);
+            }
+        }
         if (c->p.flux == 1)
             edge(wd, std::integral_constant<int, 1>());
         else if (c->p.flux == 2)
@@ -895,7 +921,42 @@ static void launch_p2_stage(dgr_ctx *c, int stage, bool count)
     if (count) c->launches += 2;
 }
 
-/* one RK stage as four kernels (buffers of stage_io) */
+template <int MODE>
+static void launch_edge_element_as(dgr_ctx *c, const double *S, const double *U, const int *wd, double *OUT, double *avg,
+                                   int stage)
+{
+    launch_dep(c->p.wet_dry ? k_edge_element<MODE, true> : k_edge_element<MODE, false>, blocks(c->ne, 32), 96, c->stream,
+               mesh_dev(c), S, U, wd, c->bzeta, c->bqn, c->flux, OUT, avg, c->clk, stage, 2 * stage, c->p.g);
+}
+
+void launch_edge_element(dgr_ctx *c, int mode, const double *S, const double *U, const int *wd, double *OUT, double *avg,
+                         int stage)
+{
+    switch (mode) {
+    case MODE_STAGE1: launch_edge_element_as<MODE_STAGE1>(c, S, U, wd, OUT, avg, stage); break;
+    case MODE_STAGE2: launch_edge_element_as<MODE_STAGE2>(c, S, U, wd, OUT, avg, stage); break;
+    case MODE_RK3_2: launch_edge_element_as<MODE_RK3_2>(c, S, U, wd, OUT, avg, stage); break;
+    default: launch_edge_element_as<MODE_RK3_3>(c, S, U, wd, OUT, avg, stage);
+    }
+}
+
+/* the second stage of SSP(3,3) updates its input in place: its elements wait for all edges */
+static bool edges_with_elements(const dgr_ctx *c, const StageIO &io) { return edges_with_elements(c) && io.S != io.OUT; }
+
+/* kernels of one RK stage at p = 1 */
+static int kernels_per_stage(const dgr_ctx *c, int stage)
+{
+    return 4 - edges_with_elements(c, stage_io(c, stage)) - limiter_folds_nodes(c);
+}
+/* kernels of a step's RK stages */
+static int kernels_of_stages(const dgr_ctx *c)
+{
+    int n = 0;
+    for (int st = 0; st < c->p.rk_stages; ++st) n += c->p.order == 2 ? 2 : kernels_per_stage(c, st);
+    return n;
+}
+
+/* one RK stage as two to four kernels (buffers of stage_io) */
 void launch_stage(dgr_ctx *c, int stage, bool count)
 {
     if (c->p.order == 2) {
@@ -906,11 +967,14 @@ void launch_stage(dgr_ctx *c, int stage, bool count)
     const StageIO io = stage_io(c, stage);
     int *dl = c->p.record_decisions ? c->dec + (size_t)(2 * stage) * c->ne : nullptr;
     int *dp = c->p.record_decisions ? c->dec + (size_t)(2 * stage + 1) * c->ne : nullptr;
-    {
-        NvtxRange r("k_edge_flux");
-        launch_edge(c, io.S, io.wd_in, stage, 2 * stage);
-    }
-    {
+    if (edges_with_elements(c, io)) {
+        NvtxRange r("k_edge_element");
+        launch_edge_element(c, io.mode, io.S, c->U, io.wd_in, io.OUT, c->avg, stage);
+    } else {
+        {
+            NvtxRange r("k_edge_flux");
+            launch_edge(c, io.S, io.wd_in, stage, 2 * stage);
+        }
         NvtxRange r("k_element");
         switch (io.mode) {
         case MODE_STAGE1: launch_element<MODE_STAGE1>(c, io.S, io.wd_in, io.OUT); break;
@@ -919,18 +983,23 @@ void launch_stage(dgr_ctx *c, int stage, bool count)
         default: launch_element<MODE_RK3_3>(c, io.S, io.wd_in, io.OUT);
         }
     }
-    {
-        NvtxRange r("k_node_bounds");
-        launch_dep(k_node_bounds, blocks(c->nn, DGR_NODE_BS), DGR_NODE_BS, c->stream, mesh_dev(c), c->avg, c->bounds);
-    }
-    {
+    if (limiter_folds_nodes(c)) {
+        NvtxRange r("k_fold_limit");
+        launch_dep(wd ? k_fold_limit<true, true, true> : k_fold_limit<true, false, false>, blocks(c->ne, 64), 64,
+                   c->stream, mesh_dev(c), io.OUT, c->avg, io.wd_in, io.wd_out, c->clk, c->p.H0, c->p.VELZERO,
+                   2 * stage + 1, dl, dp);
+    } else {
+        {
+            NvtxRange r("k_node_bounds");
+            launch_dep(k_node_bounds, blocks(c->nn, DGR_NODE_BS), DGR_NODE_BS, c->stream, mesh_dev(c), c->avg, c->bounds);
+        }
         NvtxRange r("k_limit");
         if (wd)
             launch_limit<true, true, true>(c, io.OUT, io.wd_in, io.wd_out, 2 * stage + 1, dl, dp);
         else
             launch_limit<true, false, false>(c, io.OUT, io.wd_in, io.wd_out, 2 * stage + 1, dl, dp);
     }
-    if (count) c->launches += 4; /* edge flux, element, node bounds, limiter */
+    if (count) c->launches += kernels_per_stage(c, stage);
 }
 
 void launch_wd_refresh(dgr_ctx *c)
@@ -1050,7 +1119,7 @@ static int kernels_per_step(const dgr_ctx *c)
     const int ns = c->p.rk_stages;
     const int rec = c->gauge_n ? 1 : 0;
     if (c->p.order == 2) return 1 + 2 * ns + rec;
-    return rec + (c->fusion == 2 ? 1 : (c->fusion == 1 ? 1 + ns : 1 + 4 * ns));
+    return rec + (c->fusion == 2 ? 1 : (c->fusion == 1 ? 1 + ns : 1 + kernels_of_stages(c)));
 }
 
 int decode_err(unsigned long long key, int *code, int *index, int *step)
@@ -1143,7 +1212,7 @@ extern "C" int dgr_step(dgr_ctx *c, double time, double dt, double *max_lambda)
     launch_wd_refresh(c);
     if (c->stage_graph_exec) {
         CK(cudaGraphLaunch(c->stage_graph_exec, s));
-        c->launches += (long long)c->p.rk_stages * (c->p.order == 2 ? 2 : 4);
+        c->launches += kernels_of_stages(c);
     } else {
         for (int st = 0; st < c->p.rk_stages; ++st) launch_stage(c, st, true);
     }

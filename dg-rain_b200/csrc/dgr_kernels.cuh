@@ -64,7 +64,9 @@ DGR_DEV T ldm(const T *p)
  * finishes.  pdl_wait returns once every earlier kernel of the stream has completed and its
  * writes are visible; before it a kernel may only touch what no kernel of a step writes (the
  * mesh).  pdl_trigger, after the wait, lets the next kernel's blocks start the same way.
- * Without the launch attribute both do nothing.  Measured together
+ * Without the launch attribute both do nothing.  Such a kernel takes the arrays it shares with
+ * others without __restrict__: a load through a restricted pointer may be moved above the wait.
+ * Measured together
  * with the merge of a step's two clock kernels and kGraphSteps (passes of 60 steps on 1,600
  * triangles and 100 on 200k): 3.36 -> 2.97 ms and 23.6 -> 22.5 ms. */
 DGR_DEV void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -186,13 +188,29 @@ __device__ __noinline__ double edge_item_plain(const MeshDev &m, const double *S
     return edge_flux_item<WD, false, FT>(m, S, wd, bzeta, bqn, flux, clk, phase, g, i);
 }
 
+/* Fhat.n of both sides of edge i */
+struct StoreFlux {
+    double *flux;
+    int lf, i;
+    DGR_DEV void operator()(const double fin[3], const double fex[3]) const
+    {
+        flux[i] = fin[0];
+        flux[lf + i] = fin[1];
+        flux[2 * lf + i] = fin[2];
+        flux[3 * lf + i] = fex[0];
+        flux[4 * lf + i] = fex[1];
+        flux[5 * lf + i] = fex[2];
+    }
+};
+
 /* The edge from its traces on: (zi, qxi, qyi) of the in side, (ze, qxe, qye) of the other side
- * (of the in side itself at a wall), the sides' wet/dry flags. */
-template <bool WD, bool COH, int FT, bool RCP>
+ * (of the in side itself at a wall), the sides' wet/dry flags.  store(fin, fex) takes the
+ * fluxes, unless the edge is redone with plain divisions, which writes them to `flux`. */
+template <bool WD, bool COH, int FT, bool RCP, class Store>
 DGR_DEV double edge_from_traces(const MeshDev &m, const double *S, const int *wd, const double *bzeta,
                                 const double *bqn, double *flux, DevClock *clk, DevClock *ck, int phase, double g,
                                 int i, int bd, bool wall, double nx, double ny, double z_edge, double zi, double qxi,
-                                double qyi, double ze, double qxe, double qye, int wdi, int wde)
+                                double qyi, double ze, double qxe, double qye, int wdi, int wde, const Store &store)
 {
     if (bd)
         ghost_state<double>(bd, nx, ny, zi, qxi, qyi, ldm<COH>(&bzeta[i]), ldm<COH>(&bqn[i]), 0.0, ze, qxe, qye);
@@ -210,13 +228,7 @@ DGR_DEV double edge_from_traces(const MeshDev &m, const double *S, const int *wd
                                     FT >= 0 ? FT : m.flux);
     }
     if (code) atomicMin(&ck->err, err_key(ldm<COH>(&ck->step), phase, code, i - ck->ed_off));
-    const int lf = m.ldF;
-    flux[i] = fin[0];
-    flux[lf + i] = fin[1];
-    flux[2 * lf + i] = fin[2];
-    flux[3 * lf + i] = fex[0];
-    flux[4 * lf + i] = fex[1];
-    flux[5 * lf + i] = fex[2];
+    store(fin, fex);
     return lam >= 0.0 ? lam : 0.0; /* NaN speeds are reported through the flux check */
 }
 
@@ -240,7 +252,7 @@ DGR_DEV double edge_flux_item(const MeshDev &m, const double *S, const int *wd, 
         m, S, wd, bzeta, bqn, flux, clk, ck, phase, g, i, (info >> 4) & 7, el_in == el_ex, m.e_geo[i],
         m.e_geo[m.ldF + i], m.e_geo[2 * m.ldF + i], st(k_in, el_in), st(3 + k_in, el_in), st(6 + k_in, el_in),
         st(k_ex, el_ex), st(3 + k_ex, el_ex), st(6 + k_ex, el_ex), WD ? ldm<COH>(&wd[el_in]) : 1,
-        WD ? ldm<COH>(&wd[el_ex]) : 1);
+        WD ? ldm<COH>(&wd[el_ex]) : 1, StoreFlux{flux, m.ldF, i});
 }
 
 /* Max of the wave speed per scenario: one atomic per block when the block's edges all
@@ -362,7 +374,8 @@ __global__ void __launch_bounds__(DGR_EDGE_BS, DGR_MINB_EDGE)
                                edge_from_traces<WD, false, FT, FT == 0>(
                                    m, S, wd, bzeta, bqn, flux, clk, ck, phase, g, i, kind & 7, (kind & 8) != 0,
                                    tr[b][6][t], tr[b][7][t], tr[b][8][t], tr[b][0][t], tr[b][1][t], tr[b][2][t],
-                                   tr[b][3][t], tr[b][4][t], tr[b][5][t], WD ? fl[b][0][t] : 1, WD ? fl[b][1][t] : 1));
+                                   tr[b][3][t], tr[b][4][t], tr[b][5][t], WD ? fl[b][0][t] : 1, WD ? fl[b][1][t] : 1,
+                                   StoreFlux{flux, lf, i}));
         }
         kind = next;
     }
@@ -407,23 +420,16 @@ __device__ __noinline__ void element_item_plain(const MeshDev &m, const double *
     element_item<MODE, COH, false>(m, S, U, wd, flux, out, avg, clk, g, el);
 }
 
+/* The element from its gathered edge fluxes on. */
 template <int MODE, bool COH, bool RCP>
-DGR_DEV void element_item(const MeshDev &m, const double *S, const double *U, const int *wd, const double *flux,
-                          double *out, double *avg, const DevClock *clk, double g, int el)
+DGR_DEV void element_from_flux(const MeshDev &m, const double *S, const double *U, const int *wd, const double *flux,
+                               double *out, double *avg, const DevClock *clk, const DevClock *ck, double g, int el,
+                               const double F[3][3])
 {
-    const DevClock *ck = clk + (m.el_sid ? m.el_sid[el] : 0);
     const int ld = m.ldE;
-    const int ee[3] = {m.elem_edge[el], m.elem_edge[ld + el], m.elem_edge[2 * ld + el]};
-    if (!COH) {
-        pdl_wait();
-        pdl_trigger();
-    }
-    if (ldm<COH>(&ck->done)) return;
     const double rain = ck->rain;
     const double *G = m.geo + geo_offset(el, ld);
     const int gs = geo_stride(ld);
-    double F[3][3];
-    if (!gather_flux<COH>(m, flux, el, ee, F)) return;
     double zr[3], qxr[3], qyr[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -452,6 +458,23 @@ DGR_DEV void element_item(const MeshDev &m, const double *S, const double *U, co
     }
 }
 
+template <int MODE, bool COH, bool RCP>
+DGR_DEV void element_item(const MeshDev &m, const double *S, const double *U, const int *wd, const double *flux,
+                          double *out, double *avg, const DevClock *clk, double g, int el)
+{
+    const DevClock *ck = clk + (m.el_sid ? m.el_sid[el] : 0);
+    const int ld = m.ldE;
+    const int ee[3] = {m.elem_edge[el], m.elem_edge[ld + el], m.elem_edge[2 * ld + el]};
+    if (!COH) {
+        pdl_wait();
+        pdl_trigger();
+    }
+    if (ldm<COH>(&ck->done)) return;
+    double F[3][3];
+    if (!gather_flux<COH>(m, flux, el, ee, F)) return;
+    element_from_flux<MODE, COH, RCP>(m, S, U, wd, flux, out, avg, clk, ck, g, el, F);
+}
+
 template <int MODE, int BS>
 __global__ void __launch_bounds__(BS, DGR_ELEMENT_THREADS_PER_SM / BS) k_element(const __grid_constant__ MeshDev m, const double *S,
                                                           const double *U, const int *wd,
@@ -463,6 +486,94 @@ __global__ void __launch_bounds__(BS, DGR_ELEMENT_THREADS_PER_SM / BS) k_element
     prefetch_geometry(m, blockIdx.x * BS, min(BS, m.ne - blockIdx.x * BS));
     const int el = blockIdx.x * BS + threadIdx.x;
     if (el < m.ne) element_item<MODE>(m, S, U, wd, flux, out, avg, clk, g, el);
+}
+
+/* Edges (Roe flux) and elements of a mesh that leaves most of the chip idle, in one launch: a
+ * block takes 32 elements, warp k computes the flux of their local edges k (an interior edge is
+ * computed from both sides), and warp 0 goes on with the elements from shared memory.  On such
+ * meshes a launch is a chain of dependent latencies, and the second flux of an edge costs
+ * nothing that was in use: 1,600 triangles 42.7 -> 36.8 us per step, 8,000 46.0 -> 45.0
+ * (DGR_EDGE_ELEMENT_MAX).  S and out are different arrays. */
+template <int MODE, bool WD>
+__global__ void __launch_bounds__(96, 5)
+    k_edge_element(const __grid_constant__ MeshDev m, const double *S, const double *U, const int *wd,
+                   const double *bzeta, const double *bqn, double *flux, double *out, double *avg, DevClock *clk,
+                   int lam_slot, int phase, double g)
+{
+    __shared__ double Fs[9][32];
+    __shared__ double fastest[3];
+    const int base = blockIdx.x * 32, lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+    const int el = base + lane, ld = m.ldE, lf = m.ldF;
+    prefetch_geometry(m, base, min(32, m.ne - base));
+    const bool valid = el < m.ne;
+    int i = 0, side = 0, el_in = 0, el_ex = 0, info = -1;
+    double nx = 0, ny = 0, z_edge = 0;
+    if (valid) {
+        const int ee = m.elem_edge[k * ld + el];
+        i = ee >> 1;
+        side = ee & 1;
+        if (index_ok(m, i, m.nf, KID_ELEMENT, el)) {
+            el_in = m.e_in[i];
+            el_ex = m.e_ex[i];
+            info = m.e_info[i];
+            nx = m.e_geo[i];
+            ny = m.e_geo[lf + i];
+            z_edge = m.e_geo[2 * lf + i];
+            if (!edge_indices_ok(m, i, el_in, el_ex, info)) info = -1;
+        }
+    }
+    const int sid = (valid && m.el_sid) ? m.el_sid[el] : 0;
+    const bool one_scenario = !m.el_sid || m.el_sid[base] == m.el_sid[min(base + 31, m.ne - 1)];
+    DevClock *ck = clk + sid;
+    pdl_wait();
+    pdl_trigger();
+    const bool live = valid && !ck->done;
+    double lam = 0.0;
+#pragma unroll
+    for (int v = 0; v < 3; ++v) Fs[3 * v + k][lane] = 0.0;
+    if (live && info >= 0) {
+        const int k_in = info & 3, k_ex = (info >> 2) & 3;
+        bool stored = false;
+        double f[3];
+        const auto own_side = [&](const double fin[3], const double fex[3]) {
+#pragma unroll
+            for (int v = 0; v < 3; ++v) {
+                f[v] = side ? fex[v] : fin[v];
+                flux[(3 * side + v) * lf + i] = f[v];
+            }
+            stored = true;
+        };
+        lam = edge_from_traces<WD, false, 0, true>(
+            m, S, wd, bzeta, bqn, flux, clk, ck, phase, g, i, (info >> 4) & 7, el_in == el_ex, nx, ny, z_edge,
+            S[k_in * ld + el_in], S[(3 + k_in) * ld + el_in], S[(6 + k_in) * ld + el_in], S[k_ex * ld + el_ex],
+            S[(3 + k_ex) * ld + el_ex], S[(6 + k_ex) * ld + el_ex], WD ? wd[el_in] : 1, WD ? wd[el_ex] : 1, own_side);
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+            if (!stored) f[v] = flux[(3 * side + v) * lf + i];
+            Fs[3 * v + k][lane] = side ? -f[v] : f[v];
+        }
+        if (side) lam = 0.0; /* the "in" side's thread reports it */
+    }
+    if (one_scenario) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) lam = fmax(lam, __shfl_xor_sync(0xffffffffu, lam, o));
+        if (lane == 0) fastest[k] = lam;
+    } else if (lam > 0.0) {
+        atomicMax(&ck->lam_bits[lam_slot], (unsigned long long)__double_as_longlong(lam));
+    }
+    __syncthreads();
+    if (threadIdx.x == 32 && one_scenario) {
+        lam = fmax(fmax(fastest[0], fastest[1]), fastest[2]);
+        if (lam > 0.0) atomicMax(&ck->lam_bits[lam_slot], (unsigned long long)__double_as_longlong(lam));
+    }
+    if (k == 0 && live) {
+        double F[3][3];
+#pragma unroll
+        for (int v = 0; v < 3; ++v)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) F[v][j] = Fs[3 * v + j][lane];
+        element_from_flux<MODE, false, true>(m, S, U, wd, flux, out, avg, clk, ck, g, el, F);
+    }
 }
 
 /* ------------------------------------------------------------------ nodes ---- */
@@ -538,26 +649,88 @@ static __global__ void __launch_bounds__(256) k_wd_status(MeshDev m, const doubl
 
 /* ---------------------------------------------------------- limit + PDop ---- */
 
+/* Node bounds of an element's three vertices taken from the element means directly (node_item's
+ * comparisons in its order, the first kFirst elements around a node prepared ahead; a shorter
+ * list repeats its first element, which changes no maximum). */
+struct NodeFold {
+    static constexpr int kFirst = 6;
+    int b[3], e[3], id[3][kFirst];
+    double mx[3][3], mn[3][3];
+    /* the elements around the vertices (mesh data only) */
+    DGR_DEV bool around(const MeshDev &m, const int nd[3], int el)
+    {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            b[k] = m.n2e_ptr[nd[k]];
+            e[k] = m.n2e_ptr[nd[k] + 1];
+            if (!(index_ok(m, b[k], 3 * m.ne + 1, KID_NODE, el) && index_ok(m, e[k], 3 * m.ne + 1, KID_NODE, el) &&
+                  index_ok(m, e[k] - b[k], 3 * m.ne + 1, KID_NODE, el)))
+                return false;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int j = 0; j < kFirst; ++j) {
+                id[k][j] = m.n2e[b[k] + j < e[k] ? b[k] + j : b[k]];
+                if (!index_ok(m, id[k][j], m.ne, KID_NODE, el)) return false;
+            }
+        return true;
+    }
+    DGR_DEV void add(const MeshDev &m, const double *avg, int k, int el)
+    {
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+            const double a = avg[v * m.ldE + el];
+            if (a < mn[v][k]) mn[v][k] = a;
+            if (a > mx[v][k]) mx[v][k] = a;
+        }
+    }
+    DGR_DEV void take(const MeshDev &m, const double *avg, int el)
+    {
+#pragma unroll
+        for (int v = 0; v < 3; ++v)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                mx[v][k] = -99999;
+                mn[v][k] = 99999;
+            }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int j = 0; j < kFirst; ++j) add(m, avg, k, id[k][j]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            for (int j = b[k] + kFirst; j < e[k]; ++j) {
+                const int next = m.n2e[j];
+                if (index_ok(m, next, m.ne, KID_NODE, el)) add(m, avg, k, next);
+            }
+    }
+};
+
 /*
  * One element: vertex-based limiter and positive-depth operator (limit_core), then the
  * wet/dry status (2DCode/wetDry2D.c:16-60) that the reference calls next.  wd_in is the
  * status the element had; the new status goes to wd_out.
  */
-template <bool LIMIT, bool PDOP, bool STATUS, bool COH = false>
+template <bool LIMIT, bool PDOP, bool STATUS, bool COH = false, bool FOLD = false>
 DGR_DEV void limit_item(const MeshDev &m, double *S, const double *bounds, const int *wd_in, int *wd_out,
                         DevClock *clk, double h0, double velzero, int phase, int *dec_limit, int *dec_pdop, int el)
 {
     DevClock *ck = clk + (m.el_sid ? m.el_sid[el] : 0);
     const int ld = m.ldE;
     const int nd[3] = {m.el2v[el], m.el2v[ld + el], m.el2v[2 * ld + el]};
+    const bool nodes_ok = index_ok(m, nd[0], m.nn, KID_LIMIT, el) && index_ok(m, nd[1], m.nn, KID_LIMIT, el) &&
+                          index_ok(m, nd[2], m.nn, KID_LIMIT, el);
+    NodeFold fold;
+    bool fold_ok = true;
+    if (FOLD && nodes_ok) fold_ok = fold.around(m, nd, el);
     if (!COH) {
         pdl_wait();
         pdl_trigger();
     }
     if (ldm<COH>(&ck->done)) return;
-    if (!(index_ok(m, nd[0], m.nn, KID_LIMIT, el) && index_ok(m, nd[1], m.nn, KID_LIMIT, el) &&
-          index_ok(m, nd[2], m.nn, KID_LIMIT, el)))
-        return;
+    if (!nodes_ok || !fold_ok) return;
+    if (FOLD) fold.take(m, bounds, el);
     const double zn[3] = {m.zn[nd[0]], m.zn[nd[1]], m.zn[nd[2]]};
     double w[3][3];
 #pragma unroll
@@ -565,7 +738,8 @@ DGR_DEV void limit_item(const MeshDev &m, double *S, const double *bounds, const
 #pragma unroll
         for (int k = 0; k < 3; ++k) w[v][k] = ldm<COH>(&S[(3 * v + k) * ld + el]);
     const int lb = m.ldN;
-    const auto bnd = [bounds, lb, &nd](int v, int k, int is_min) {
+    const auto bnd = [bounds, lb, &nd, &fold](int v, int k, int is_min) {
+        if constexpr (FOLD) return is_min ? fold.mn[v][k] : fold.mx[v][k];
         return ldm<COH>(&bounds[(3 * is_min + v) * lb + nd[k]]);
     };
     LimitDecisions dec;
@@ -592,6 +766,20 @@ __global__ void __launch_bounds__(BS, DGR_LIMIT_THREADS_PER_SM / BS) k_limit(con
     const int el = blockIdx.x * BS + threadIdx.x;
     if (el < m.ne)
         limit_item<LIMIT, PDOP, STATUS>(m, S, bounds, wd_in, wd_out, clk, h0, velzero, phase, dec_limit, dec_pdop, el);
+}
+
+/* The limiter of a mesh that leaves most of the chip idle: it takes the node bounds from the
+ * means itself, 54 gathers in flight at once instead of a launch of k_node_bounds and the 18 of
+ * its results (figures at DGR_FOLD_LIMIT_MAX). */
+template <bool LIMIT, bool PDOP, bool STATUS>
+__global__ void __launch_bounds__(64, 8) k_fold_limit(const __grid_constant__ MeshDev m, double *S, const double *avg,
+                                                      const int *wd_in, int *wd_out, DevClock *clk, double h0,
+                                                      double velzero, int phase, int *dec_limit, int *dec_pdop)
+{
+    const int el = blockIdx.x * 64 + threadIdx.x;
+    if (el < m.ne)
+        limit_item<LIMIT, PDOP, STATUS, false, true>(m, S, avg, wd_in, wd_out, clk, h0, velzero, phase, dec_limit,
+                                                     dec_pdop, el);
 }
 
 /* ------------------------------------------------------------------ clock ---- */
