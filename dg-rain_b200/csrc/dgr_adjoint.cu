@@ -486,25 +486,26 @@ static void reverse_stage(dgr_ctx *c, int j, int n, int stage)
     c->launches += 4;
 }
 
-/* planar [3 nm][ldE] -> the reference layout zeta/Qx/Qy[nm*el+k] on the host */
-static int to_reference_layout(dgr_ctx *c, const double *planar, double *zeta, double *Qx, double *Qy)
+/* the gradient to the host, the initial state's part in the reference layout
+ * zeta/Qx/Qy[nm*el+k] */
+static int download_gradient(dgr_ctx *c, double *n_el, double *z, double *zeta, double *Qx, double *Qy)
 {
-    if (!zeta && !Qx && !Qy) return DGR_OK;
+    const AdjointState *a = c->adj;
     const size_t n3 = (size_t)c->nm * c->ne;
-    double *tmp = nullptr;
-    int r = dalloc(&tmp, 3 * n3);
-    if (r) return r;
-    k_planar_to_aos_nm<<<blocks(c->ne, 256), 256, 0, c->stream>>>(c->ne, c->ldE, c->nm, planar, tmp, tmp + n3,
-                                                                   tmp + 2 * n3);
-    c->launches++;
-    std::vector<double> h(3 * n3);
-    cudaError_t e = cudaMemcpyAsync(h.data(), tmp, 3 * n3 * 8, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaFree(tmp);
-    CK(e);
-    if (zeta) memcpy(zeta, h.data(), n3 * 8);
-    if (Qx) memcpy(Qx, h.data() + n3, n3 * 8);
-    if (Qy) memcpy(Qy, h.data() + 2 * n3, n3 * 8);
+    double *st = c->W; /* staging, as for the state: W is free between steps */
+    if (zeta || Qx || Qy) {
+        k_planar_to_aos_nm<<<blocks(c->ne, 256), 256, 0, c->stream>>>(c->ne, c->ldE, c->nm, a->lamU, st, st + n3,
+                                                                       st + 2 * n3);
+        c->launches++;
+        CK(cudaGetLastError());
+    }
+    const HostCopy down[5] = {{n_el, a->nbar, n_el ? (size_t)c->ne * 8 : 0},
+                              {z, a->zbar, z ? (size_t)c->nn * 8 : 0},
+                              {zeta, st, zeta ? n3 * 8 : 0},
+                              {Qx, st + n3, Qx ? n3 * 8 : 0},
+                              {Qy, st + 2 * n3, Qy ? n3 * 8 : 0}};
+    CK(host_copies(c, down, 5, true));
+    CK(cudaStreamSynchronize(c->stream));
     return DGR_OK;
 }
 
@@ -575,9 +576,7 @@ extern "C" int dgr_adjoint_backward(dgr_ctx *c, double *grad_n_el, double *grad_
     if (r) return r;
     r = first_error(c);
     if (r) return r;
-    if (grad_n_el) CK(cudaMemcpy(grad_n_el, a->nbar, (size_t)c->ne * 8, cudaMemcpyDeviceToHost));
-    if (grad_z) CK(cudaMemcpy(grad_z, a->zbar, (size_t)c->nn * 8, cudaMemcpyDeviceToHost));
-    r = to_reference_layout(c, a->lamU, grad_zeta0, grad_Qx0, grad_Qy0);
+    r = download_gradient(c, grad_n_el, grad_z, grad_zeta0, grad_Qx0, grad_Qy0);
     if (r) return r;
     c->wd_fresh = 0; /* the context state is the last recomputed one */
     return DGR_OK;

@@ -84,11 +84,12 @@ static void release(dgr_ctx *c)
                     c->e_ex, c->e_info, c->n2e_ptr, c->n2e, c->bnd_edges, c->bnd_type, c->bnd_sid, c->bdry,
                     c->el_sid, c->ed_sid, c->e_geo, c->geo, c->U, c->W, c->flux, c->avg, c->bounds, c->bzeta,
                     c->bqn, c->bstage, c->wdA, c->wdB, c->wdC, c->dec, c->bar, c->clk, c->p2g,
-                    c->gauge_el, c->gauge_sid, c->gauge_w, c->gauge_series};
+                    c->gauge_el, c->gauge_sid, c->gauge_w, c->gauge_series, c->rhs_stage};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     adjoint_release(c);
     coupling_release(c);
+    stager_release(c);
     if (c->h_clk) cudaFreeHost(c->h_clk);
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->ev0) cudaEventDestroy(c->ev0);
@@ -555,6 +556,7 @@ static int create_impl(int nscen, const dgr_mesh_view *views, const dgr_scenario
     c->wd_fresh = 0;
     c->wd_stepped = 0;
     set_carveouts(c);
+    stager_create(c);
     *out = c;
     return DGR_OK;
 }
@@ -674,9 +676,11 @@ int upload_scenarios(dgr_ctx *c, int s0, int s1, const double *zeta, const doubl
     const size_t n3 = (size_t)c->nm * n; /* coefficients per variable */
     double *st = c->W; /* staging: W is free between steps */
     cudaStream_t s = c->stream;
-    CK(cudaMemcpyAsync(st, zeta, n3 * 8, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(st + n3, Qx, n3 * 8, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(st + 2 * n3, Qy, n3 * 8, cudaMemcpyHostToDevice, s));
+    const HostCopy up[4] = {{(void *)zeta, st, n3 * 8},
+                            {(void *)Qx, st + n3, n3 * 8},
+                            {(void *)Qy, st + 2 * n3, n3 * 8},
+                            {(void *)WD, c->wdA + c->el_off[s0], WD ? (size_t)n * 4 : 0}};
+    CK(host_copies(c, up, 4, false));
     k_aos_to_planar_nm<<<blocks(n, 256), 256, 0, s>>>(n, c->ldE, c->nm, st, st + n3, st + 2 * n3,
                                                       c->U + c->el_off[s0]);
     c->launches++;
@@ -686,7 +690,6 @@ int upload_scenarios(dgr_ctx *c, int s0, int s1, const double *zeta, const doubl
             if (k < s0 || k >= s1)
                 CK(cudaMemcpyAsync(c->wdA + c->el_off[k], wd_after_step(c) + c->el_off[k],
                                    (size_t)(c->el_off[k + 1] - c->el_off[k]) * 4, cudaMemcpyDeviceToDevice, s));
-    if (WD) CK(cudaMemcpyAsync(c->wdA + c->el_off[s0], WD, (size_t)n * 4, cudaMemcpyHostToDevice, s));
     CK(cudaStreamSynchronize(s));
     /* clear the scenarios' error words and run state */
     int r = read_clock(c);
@@ -719,12 +722,11 @@ static int download_slice(dgr_ctx *c, int sc, double *zeta, double *Qx, double *
     k_planar_to_aos_nm<<<blocks(n, 256), 256, 0, s>>>(n, c->ldE, c->nm, c->U + c->el_off[sc], st, st + n3,
                                                       st + 2 * n3);
     c->launches++;
-    CK(cudaMemcpyAsync(zeta, st, n3 * 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(Qx, st + n3, n3 * 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(Qy, st + 2 * n3, n3 * 8, cudaMemcpyDeviceToHost, s));
-    if (WD)
-        CK(cudaMemcpyAsync(WD, (c->wd_stepped ? wd_after_step(c) : c->wdA) + c->el_off[sc], (size_t)n * 4,
-                           cudaMemcpyDeviceToHost, s));
+    const HostCopy down[4] = {{zeta, st, n3 * 8},
+                              {Qx, st + n3, n3 * 8},
+                              {Qy, st + 2 * n3, n3 * 8},
+                              {WD, (c->wd_stepped ? wd_after_step(c) : c->wdA) + c->el_off[sc], WD ? (size_t)n * 4 : 0}};
+    CK(host_copies(c, down, 4, true));
     CK(cudaStreamSynchronize(s));
     return DGR_OK;
 }
@@ -1253,15 +1255,18 @@ extern "C" int dgr_compute_L(dgr_ctx *c, double time, double *rz, double *rqx, d
     CK(cudaGetLastError());
     if (rz && rqx && rqy) {
         const size_t n3 = (size_t)c->nm * c->ne;
-        double *tmp = nullptr; /* stream-ordered staging for the reference layout */
-        CK(cudaMallocAsync((void **)&tmp, 3 * n3 * 8, s));
+        /* staging for the reference layout, kept: a stream-ordered allocation goes back to the
+         * system at every synchronisation */
+        if (!c->rhs_stage) {
+            const int r = dalloc(&c->rhs_stage, 3 * n3);
+            if (r) return r;
+        }
+        double *tmp = c->rhs_stage;
         k_planar_to_aos_nm<<<blocks(c->ne, 256), 256, 0, s>>>(c->ne, c->ldE, c->nm, c->W, tmp, tmp + n3,
                                                               tmp + 2 * n3);
         c->launches++;
-        CK(cudaMemcpyAsync(rz, tmp, n3 * 8, cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(rqx, tmp + n3, n3 * 8, cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(rqy, tmp + 2 * n3, n3 * 8, cudaMemcpyDeviceToHost, s));
-        CK(cudaFreeAsync(tmp, s));
+        const HostCopy down[3] = {{rz, tmp, n3 * 8}, {rqx, tmp + n3, n3 * 8}, {rqy, tmp + 2 * n3, n3 * 8}};
+        CK(host_copies(c, down, 3, true));
     }
     int r = read_clock(c);
     if (r) return r;

@@ -20,6 +20,7 @@
 
 namespace dgr {
 struct AdjointState; /* dgr_adjoint.cu */
+struct Stager;       /* dgr_transfer.cu */
 }
 
 /* last CUDA error text, per host thread (dgr_last_cuda_error) */
@@ -76,6 +77,7 @@ struct dgr_ctx {
     double *e_geo, *geo;
     /* state and work */
     double *U, *W, *flux, *avg, *bounds, *bzeta, *bqn, *bstage;
+    double *rhs_stage; /* dgr_compute_L's results in the reference layout, allocated on its first call */
     int *wdA, *wdB, *wdC; /* wet/dry flags: stage s reads buffer s, writes buffer (s+1) mod stages */
     int *dec; /* [6][ne]: limit and pdop decisions of stage 0, 1, 2 */
     unsigned *bar;
@@ -98,6 +100,7 @@ struct dgr_ctx {
     cudaGraphExec_t stage_graph_exec;
     int stage_graph_tried;            /* its capture was attempted since the last drop_graph */
     dgr::AdjointState *adj; /* discrete adjoint storage, created on first use */
+    dgr::Stager *stager;    /* threaded host copies (dgr_transfer.cu); null in a small context */
     /* gauge series recorded by the device loop (dgr_set_gauges) */
     int gauge_n, gauge_cap;
     int *gauge_el, *gauge_sid;
@@ -203,6 +206,20 @@ static inline void launch_dep(void (*kernel)(P...), unsigned grid, unsigned bloc
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
+
+namespace dgr {
+/* dgr_transfer.cu: copies between the caller's arrays and the device, in the order of the
+ * context's stream.  After host_copies returns, copies up can be used by later work on the
+ * stream and the caller's arrays are free; copies down are complete once the stream is. */
+struct HostCopy {
+    void *host, *dev;
+    size_t bytes;
+};
+constexpr int kMaxHostCopies = 8;
+cudaError_t host_copies(dgr_ctx *c, const HostCopy *p, int n, bool down);
+void stager_create(dgr_ctx *c);
+void stager_release(dgr_ctx *c);
+}  // namespace dgr
 
 /* dgr_capi.cu */
 void drop_graph(dgr_ctx *c);
