@@ -6,7 +6,7 @@
 The library is built in-tree so that it travels with the repository to the GPU host.
 
 Flags: sm_100a only; --fmad=false keeps every multiply and add a separately rounded IEEE
-operation so that the kernels reproduce the reference C step's arithmetic.
+operation so that the kernels reproduce the reference C step's arithmetic (except CONTRACTED).
 """
 from __future__ import annotations
 
@@ -31,7 +31,9 @@ NVCC_FLAGS = [
 CC_FLAGS = ["-std=c99", "-O2", "-ffp-contract=off", "-fPIC", "-Wall", "-Wextra", "-Wno-unused-parameter"]
 
 CU_SOURCES = ["dgr_capi.cu", "dgr_noalloc.cu", "dgr_adjoint.cu", "dgr_output.cu", "dgr_ingest.cu", "dgr_coupling.cu",
-              "dgr_transfer.cu"]
+              "dgr_transfer.cu", "dgr_adjoint_elements.cu"]
+# reverse kernels that recompute none of the forward step's decisions: contraction allowed
+CONTRACTED = {"dgr_adjoint_elements.cu"}
 C_SOURCES = ["dgr_host.c"]
 DEPS = ["dgr_kernels.cuh", "dgr_device.cuh", "dgr_forcing.h", "dgr_internal.cuh", "dgr_scheme.cuh",
         "dgr_dual.cuh", "dgr_reverse.cuh", "dgr_tlm.cuh", "dgr_p2.cuh", "dgr_p2_adjoint.cuh", "dgr_format.cuh", "dgr_ptr.h", os.path.join("..", "..", "include", "dgrain.h")]
@@ -81,7 +83,8 @@ def build(verbose: bool = False, ptxas_verbose: bool = False, force: bool = Fals
     for f in CU_SOURCES:
         o = os.path.join(build_dir, f + ".o")
         extra = ["-Xptxas", "-v"] if ptxas_verbose else []
-        jobs.append(([nvcc, *NVCC_FLAGS, *dflags, *extra, "-c", os.path.join(CSRC, f), "-o", o],
+        flags = [x for x in NVCC_FLAGS if not (f in CONTRACTED and x == "--fmad=false")]
+        jobs.append(([nvcc, *flags, *dflags, *extra, "-c", os.path.join(CSRC, f), "-o", o],
                      verbose or ptxas_verbose))
         objs.append(o)
     # the translation units are independent: compiled side by side

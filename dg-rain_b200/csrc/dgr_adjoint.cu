@@ -405,18 +405,7 @@ static void reverse_stage_p2(dgr_ctx *c, int j, int n, int stage)
     const int u_acc = stage < ns - 1 ? 1 : 0;
     const double g = c->p.g;
     const unsigned nb = blocks(c->ne, 128);
-#define P2_ADJ_EL(MD)                                                                                                  \
-    launch_dep(k_p2_adj_element<MD>, nb, 128, s, c->p2ref, m, c->p2g, S, lamO, lamS, a->lamU, u_acc, a->fbar, a->zvb,    \
-                                            a->nbar, c->n_el, g, dt_row(c, n))
-    if (mode == MODE_STAGE1)
-        P2_ADJ_EL(MODE_STAGE1);
-    else if (mode == MODE_STAGE2)
-        P2_ADJ_EL(MODE_STAGE2);
-    else if (mode == MODE_RK3_2)
-        P2_ADJ_EL(MODE_RK3_2);
-    else
-        P2_ADJ_EL(MODE_RK3_3);
-#undef P2_ADJ_EL
+    launch_p2_adj_element(c, mode, S, lamO, lamS, a->lamU, u_acc, a->fbar, a->zvb, a->nbar, dt_row(c, n));
     if (c->p.flux == 0)
         launch_dep(k_p2_adj_edge<0>, blocks(c->nf, 128), 128, s, c->p2ref, m, c->p2g, S, c->bzeta, c->bqn, a->fbar, a->zeb,
                                                             g);
@@ -456,18 +445,8 @@ static void reverse_stage(dgr_ctx *c, int j, int n, int stage)
         launch_dep(k_adj_limit<false>, nb, 128, s, m, seg_R(c, j, stage), seg_B(c, j, stage), lamO, a->Rbar, a->bbar,
                                               a->zvb, h0, vz);
     launch_dep(k_adj_node, blocks(c->nn, 256), 256, s, m, seg_avg(c, j, stage), a->bbar, a->bnode, a->barg);
-#define ADJ_EL(MD)                                                                                                 \
-    launch_dep(k_adj_element<MD>, nb, 128, s, m, S, wd_in, a->Rbar, a->bnode, a->barg, lamS, a->lamU, u_acc, a->fbar,   \
-                                         a->zvb, a->nbar, c->n_el, g, dt_row(c, n))
-    if (mode == MODE_STAGE1)
-        ADJ_EL(MODE_STAGE1);
-    else if (mode == MODE_STAGE2)
-        ADJ_EL(MODE_STAGE2);
-    else if (mode == MODE_RK3_2)
-        ADJ_EL(MODE_RK3_2);
-    else
-        ADJ_EL(MODE_RK3_3);
-#undef ADJ_EL
+    launch_adj_element(c, mode, S, wd_in, a->Rbar, a->bnode, a->barg, lamS, a->lamU, u_acc, a->fbar, a->zvb, a->nbar,
+                       dt_row(c, n));
 #define ADJ_EDGE(W, F) \
     launch_dep(k_adj_edge<W, F>, blocks(c->nf, DGR_ADJ_EDGE_BS), DGR_ADJ_EDGE_BS, s, m, S, wd_in, c->bzeta, c->bqn,   \
                                                                           a->fbar, lamS, a->zeb, g)

@@ -221,6 +221,13 @@ void stager_create(dgr_ctx *c);
 void stager_release(dgr_ctx *c);
 }  // namespace dgr
 
+/* dgr_adjoint_elements.cu */
+void launch_adj_element(dgr_ctx *c, int mode, const double *S, const int *wd, const double *Rbar, const double *bnode,
+                        const int *barg, double *lamS, double *lamU, int u_acc, double *fbar, double *zvb, double *nbar,
+                        const double *dt);
+void launch_p2_adj_element(dgr_ctx *c, int mode, const double *S, const double *lamO, double *lamS, double *lamU,
+                           int u_acc, double *fbar, double *zvb, double *nbar, const double *dt);
+
 /* dgr_capi.cu */
 void drop_graph(dgr_ctx *c);
 int upload_geometry(dgr_ctx *c);                 /* element geometry planes from x, y, zn, n */

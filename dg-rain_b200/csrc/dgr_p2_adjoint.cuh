@@ -171,7 +171,7 @@ DGR_HD void p2_area_rev(const P2Ref &ref, const double S[3][P2_NM], const double
         const double iH = 1.0 / H;
         const double u = uq[1] * iH, vv = uq[2] * iH;
         const double sp = sqrt(fma(u, u, vv * vv));
-        const double iP = 1.0 / pow43(H);
+        const double iP = inv_pow43(H, iH);
         const double tau = gnn * sp * iP;
         const double wj = 2.0 * ref.wq[q] * detJ;
         /* adjoints of the flux's components along r and s and of the source, then of fx, fy */
@@ -275,17 +275,13 @@ __global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_ELEMENT) k_p2_adj_element
     double cu, cs, cr;
     stage_coefficients(MODE, cu, cs, cr);
     const double rk = MODE == MODE_RHS ? 1.0 : cr * dt_n[m.el_sid ? m.el_sid[el] : 0];
-    double wb[3][P2_NM], Xb[3][P2_NM];
-#pragma unroll
-    for (int v = 0; v < 3; ++v)
-#pragma unroll
-        for (int k = 0; k < P2_NM; ++k) wb[v][k] = lamO[(P2_NM * v + k) * ld + el];
+    double Xb[3][P2_NM];
     const double idet = 1.0 / detJ;
 #pragma unroll
     for (int k = 0; k < P2_NM; ++k) {
         const double minv = idet * ref.imass[k];
 #pragma unroll
-        for (int v = 0; v < 3; ++v) Xb[v][k] = (wb[v][k] * rk) * minv;
+        for (int v = 0; v < 3; ++v) Xb[v][k] = (lamO[(P2_NM * v + k) * ld + el] * rk) * minv;
     }
     /* edge integrals: acc[v][m] -= wl F[k][gp][v] phie[k][gp][m] */
 #pragma unroll
@@ -315,7 +311,7 @@ __global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_ELEMENT) k_p2_adj_element
 #pragma unroll
         for (int k = 0; k < P2_NM; ++k) {
             s[v][k] = S[(P2_NM * v + k) * ld + el];
-            Sb[v][k] = cs * wb[v][k];
+            Sb[v][k] = 0.0;
         }
     const double zv[3] = {G[(size_t)P2G_ZV * ld], G[(size_t)(P2G_ZV + 1) * ld], G[(size_t)(P2G_ZV + 2) * ld]};
     const double gnn = G[(size_t)P2G_GNN * ld];
@@ -326,12 +322,14 @@ __global__ void __launch_bounds__(128, DGR_P2_MINB_ADJ_ELEMENT) k_p2_adj_element
     for (int v = 0; v < 3; ++v)
 #pragma unroll
         for (int k = 0; k < P2_NM; ++k) {
+            /* lamO is read once more instead of held in 36 registers over the area loop */
             const int idx = (P2_NM * v + k) * ld + el;
+            const double o = lamO[idx], sb = fma(cs, o, Sb[v][k]);
             if (MODE == MODE_STAGE1) {
-                lamS[idx] += Sb[v][k];
+                lamS[idx] += sb;
             } else {
-                lamS[idx] = Sb[v][k];
-                lamU[idx] = (u_accumulate ? lamU[idx] : 0.0) + cu * wb[v][k];
+                lamS[idx] = sb;
+                lamU[idx] = fma(cu, o, u_accumulate ? lamU[idx] : 0.0);
             }
         }
     p2_dz_rev(rx, ry, sx, sy, dzb, zvbl);

@@ -52,6 +52,16 @@ DGR_HD void normal_flux_rev(const double fb[3], double h, double u, double v, do
     zb -= pb * local_g * z_edge;
 }
 
+/* H^(-4/3) from H and 1/H, for factors of derivatives: pow43's correct rounding does not matter there */
+DGR_HD double inv_pow43(double H, double iH)
+{
+#ifdef __CUDA_ARCH__
+    return iH * rcbrt(H);
+#else
+    return iH / cbrt(H);
+#endif
+}
+
 /* Reverse of roe_flux (2DCode/numericalFlux2D.c:6-108): fhb = adjoint of Fhat.n. */
 DGR_HD void roe_flux_rev(const double fhb[3], double zeta_in, double zeta_ex, double qx_in, double qx_ex, double qy_in,
                          double qy_ex, double z_edge, double nx, double ny, double local_g, double g, RoeBar &b)
@@ -65,6 +75,7 @@ DGR_HD void roe_flux_rev(const double fhb[3], double zeta_in, double zeta_ex, do
     const double h_hat = 0.5 * (h_in + h_ex);
     const double D = s_in + s_ex;
     double u_in, u_ex, v_in, v_ex, u_hat, v_hat;
+    double ihi, ihe, iD; /* 1 / h_in, 1 / h_ex, 1 / D */
     {
         RcpDiv dv;
         const auto bi = dv.by(h_in), be = dv.by(h_ex);
@@ -73,6 +84,9 @@ DGR_HD void roe_flux_rev(const double fhb[3], double zeta_in, double zeta_ex, do
         v_in = dv.div(qy_in, bi);
         v_ex = dv.div(qy_ex, be);
         const auto bd = dv.by(D);
+        ihi = bi.y;
+        ihe = be.y;
+        iD = bd.y;
         u_hat = dv.div(u_in * s_in + u_ex * s_ex, bd);
         v_hat = dv.div(v_in * s_in + v_ex * s_ex, bd);
         if (!dv.ok) {
@@ -160,8 +174,10 @@ DGR_HD void roe_flux_rev(const double fhb[3], double zeta_in, double zeta_ex, do
     uhb += nx * unhb;
     vhb += ny * unhb;
     double uib = nx * un_in_b, vib = ny * un_in_b, ueb = nx * un_ex_b, veb = ny * un_ex_b;
-    double hib = c_in == 0.0 ? 0.0 : c_in_b * g / (2.0 * c_in);
-    double heb = c_ex == 0.0 ? 0.0 : c_ex_b * g / (2.0 * c_ex);
+    /* a side's celerity has an adjoint only where the entropy fix took its wave */
+    double hib = 0.0, heb = 0.0;
+    if (c_in_b != 0.0 && c_in != 0.0) hib = c_in_b * g / (2.0 * c_in);
+    if (c_ex_b != 0.0 && c_ex != 0.0) heb = c_ex_b * g / (2.0 * c_ex);
 
     /* c = sqrt(g h_hat), h_hat = (h_in + h_ex)/2 */
     const double hhb = c == 0.0 ? 0.0 : cb * g * ic2;
@@ -169,7 +185,6 @@ DGR_HD void roe_flux_rev(const double fhb[3], double zeta_in, double zeta_ex, do
     heb += 0.5 * hhb;
 
     /* Roe averages */
-    const double iD = 1.0 / D;
     const double Nub = uhb * iD, Nvb = vhb * iD;
     const double Db = -(uhb * u_hat + vhb * v_hat) * iD;
     uib += Nub * s_in;
@@ -177,8 +192,10 @@ DGR_HD void roe_flux_rev(const double fhb[3], double zeta_in, double zeta_ex, do
     vib += Nvb * s_in;
     veb += Nvb * s_ex;
     const double sib = Nub * u_in + Nvb * v_in + Db, seb = Nub * u_ex + Nvb * v_ex + Db;
-    hib += s_in == 0.0 ? 0.0 : sib / (2.0 * s_in);
-    heb += s_ex == 0.0 ? 0.0 : seb / (2.0 * s_ex);
+    /* 1 / s = s / h: like the other quotients that only scale derivatives, a product with the
+     * reciprocal that the forward values needed */
+    hib += s_in == 0.0 ? 0.0 : 0.5 * sib * (s_in * ihi);
+    heb += s_ex == 0.0 ? 0.0 : 0.5 * seb * (s_ex * ihe);
 
     /* physical normal fluxes */
     double zb = 0.0;
@@ -186,7 +203,6 @@ DGR_HD void roe_flux_rev(const double fhb[3], double zeta_in, double zeta_ex, do
     normal_flux_rev(p3b, h_ex, u_ex, v_ex, z_edge, nx, ny, local_g, heb, ueb, veb, zb);
 
     /* velocities */
-    const double ihi = 1.0 / h_in, ihe = 1.0 / h_ex;
     b.qxin += uib * ihi;
     b.qyin += vib * ihi;
     hib -= (uib * u_in + vib * v_in) * ihi;
@@ -566,7 +582,7 @@ DGR_HD void element_core_rev(const double wb[3][3], const double zr[3], const do
         u[e] = qxr[e] * iH[e];
         v[e] = qyr[e] * iH[e];
         sp[e] = sqrt(u[e] * u[e] + v[e] * v[e]);
-        iP[e] = 1.0 / pow43(H[e]);
+        iP[e] = inv_pow43(H[e], iH[e]);
         tau[e] = gnn[e] * sp[e] * iP[e];
     }
     const double bedx = local_g * aj * zg.gradz(0) * weight;
