@@ -9,14 +9,18 @@
  * -> 0.6 and 3.0 -> 0.9; 2 MB down 0.9 -> 0.4 (16 host cores).
  *
  * A context of at least kContextBytes of state owns the pinned chunks, streams and events (2 ms
- * to allocate).  Smaller ones (3 MB up 0.26 ms by plain copies, 0.33 by threads; down 0.30 and
- * 0.29), copies below kThreadedBytes and pinned arrays (already at the bus's speed) take plain
- * copies.
+ * to allocate).  Its copies of kThreadedBytes or more go through the threads; smaller ones (3 MB
+ * up 0.26 ms by plain copies, 0.33 by threads) only down into pages not yet there, from
+ * kFreshBytes on (2 MB 0.9 -> 0.4 ms; into resident pages 0.14 by a plain copy).  Pinned arrays
+ * are at the bus's speed already and take plain copies, as do smaller contexts.
  */
 #include <algorithm>
 #include <cstring>
 #include <new>
 #include <thread>
+
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include "dgr_internal.cuh"
 
@@ -24,7 +28,7 @@ namespace dgr {
 
 namespace {
 constexpr int kThreads = 4, kSlots = 2 * kThreads;
-constexpr size_t kChunk = 512 << 10, kThreadedBytes = 1 << 20, kContextBytes = 4 << 20;
+constexpr size_t kChunk = 512 << 10, kContextBytes = 4 << 20, kThreadedBytes = 6 << 20, kFreshBytes = 1 << 20;
 }  // namespace
 
 struct Stager {
@@ -91,6 +95,19 @@ bool is_pinned(const void *p)
     return a.type != cudaMemoryTypeUnregistered;
 }
 
+/* whether most of an array's pages (of eight looked at) are still to be provided by the kernel */
+bool is_fresh(const void *p, size_t bytes)
+{
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    int absent = 0;
+    for (int i = 0; i < 8; ++i) {
+        unsigned char in = 1;
+        void *at = (void *)(((size_t)p + bytes / 8 * i + bytes / 16) / page * page);
+        if (mincore(at, page, &in) == 0 && !(in & 1)) ++absent;
+    }
+    return absent > 4;
+}
+
 }  // namespace
 
 void stager_release(dgr_ctx *c)
@@ -135,12 +152,13 @@ cudaError_t host_copies(dgr_ctx *c, const HostCopy *p, int n, bool down)
     size_t bytes = 0;
     for (int i = 0; i < n; ++i) {
         if (!p[i].bytes) continue;
-        if (st && p[i].bytes >= kThreadedBytes / 8 && !is_pinned(p[i].host)) {
+        if (st && p[i].bytes >= kFreshBytes / 8 && !is_pinned(p[i].host)) {
             threaded[k++] = p[i];
             bytes += p[i].bytes;
         }
     }
-    const bool threads = bytes >= kThreadedBytes;
+    const bool threads = bytes >= kThreadedBytes ||
+                         (down && bytes >= kFreshBytes && is_fresh(threaded[0].host, threaded[0].bytes));
     for (int i = 0, j = 0; i < n; ++i) {
         if (!p[i].bytes) continue;
         if (j < k && threaded[j].host == p[i].host && threaded[j].dev == p[i].dev) {
