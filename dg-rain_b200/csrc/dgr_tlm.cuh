@@ -28,8 +28,8 @@
 
 /* Minimum resident blocks per SM of the reverse kernels (register caps 65536 / (threads x
  * blocks)); chosen by measurement, overridable at build time. */
-#ifndef DGR_ADJ_EDGE_BS /* threads per block of the reverse edge kernel */
-#define DGR_ADJ_EDGE_BS 256
+#ifndef DGR_ADJ_EDGE_BS /* threads per block of the reverse edge kernel (backward on 200k triangles, 20 steps: 10.04 ms at 256, 9.84 at 128) */
+#define DGR_ADJ_EDGE_BS 128
 #endif
 #ifndef DGR_ADJ_MINB_EDGE
 #define DGR_ADJ_MINB_EDGE (512 / DGR_ADJ_EDGE_BS)
