@@ -231,7 +231,7 @@ bool edges_with_elements(const dgr_ctx *c) { return c->ne <= DGR_EDGE_ELEMENT_MA
 static bool limiter_folds_nodes(const dgr_ctx *c) { return c->ne <= DGR_FOLD_LIMIT_MAX; }
 
 /* One shared-memory carveout for the p = 1 step's kernels: what four resident blocks of
- * k_edge_flux need.  An SM changes its carveout only when it is empty, so with the driver's
+ * k_edge_flux need.  An SM changes its carveout only when it is empty, so with CUDA's
  * choice per kernel (least for the others) no block of the next kernel starts while the edge
  * kernel or the one before it drains: 24k triangles 59.6 against 57.4 us per step, 200k 168.7
  * against 166.5; the whole of it taken from L1 costs more (24k 62.2, 200k 195). */

@@ -13,7 +13,8 @@
  *   avg, bounds       planar [3][ldE] element means; planar [6][ldN] node max/min
  *
  * Per RK stage: edge flux -> element RHS + RK update -> node bounds -> limiter + PDop +
- * wet/dry status.  Every kernel has one thread per edge, element or node; no atomics
+ * wet/dry status (small meshes: fewer launches, k_edge_element and k_fold_limit).  Every item
+ * (edge, element or node) is one thread's; no atomics
  * touch the data path (the edge flux is stored once per edge and gathered by both
  * elements), only the max wave speed and the first-error word are reduced atomically.
  */

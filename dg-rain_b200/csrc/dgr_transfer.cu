@@ -1,7 +1,7 @@
 /*
  * Copies between a caller's pageable arrays and the device.
  *
- * The driver moves pageable memory through one thread: 11 GB/s up, and down into pages the
+ * CUDA moves pageable memory through one thread: 11 GB/s up, and down into pages the
  * caller has just allocated (every result array of the Python package) 4-5 GB/s, most of it
  * the kernel clearing pages.  Here kThreads threads move parts of the copy, each through two
  * pinned chunks of its own, so that pages are cleared and chunks copied side by side while the
