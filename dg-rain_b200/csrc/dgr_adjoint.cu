@@ -296,7 +296,7 @@ extern "C" int dgr_adjoint_forward(dgr_ctx *c, const double *zeta, const double 
         c->launches += 2;
     }
     k_misfit_sum<<<1, 32, 0, s>>>(a->resid, nullptr, (long long)a->nsteps * a->ng, 0, a->sums);
-    k_clock_finish<<<blocks(nsc, 128), 128, 0, s>>>(c->clk, nsc, phys(c));
+    k_clock_finish<<<blocks(nsc, 128), 128, 0, s>>>(c->clk, nsc, phys(c), nullptr);
     c->launches += 2;
     CK(cudaGetLastError());
     CK(cudaEventRecord(c->ev1, s));

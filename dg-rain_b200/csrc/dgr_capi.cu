@@ -1088,6 +1088,9 @@ static cudaError_t launch_fused(dgr_ctx *c, int stage_begin, int stage_end, int 
     }
 }
 
+/* the barrier's time-out flag under a schedule with barriers (run_impl clears it), else null */
+static const unsigned *barrier_timeout(const dgr_ctx *c) { return c->fusion ? c->bar + 2 : nullptr; }
+
 /* One step of the device loop with the current schedule. */
 static cudaError_t launch_step(dgr_ctx *c)
 {
@@ -1099,7 +1102,7 @@ static cudaError_t launch_step(dgr_ctx *c)
         if (e != cudaSuccess) return e;
     } else {
         launch_dep(k_clock_begin, 1, 256, s, c->clk, c->nscen, p, c->bnd_edges, c->bnd_type, c->bnd_sid, c->nbnd,
-                                        c->bzeta, c->bqn);
+                                        c->bzeta, c->bqn, barrier_timeout(c));
         for (int st = 0; st < ns; ++st) {
             if (c->fusion == 1 && c->p.order == 1) {
                 cudaError_t e = launch_fused(c, st, st + 1, 0);
@@ -1423,7 +1426,7 @@ static int run_impl(dgr_ctx *c, int nsteps, const double *final_time, double *ti
         }
     }
     c->launches += (long long)nsteps * kernels_per_step(c);
-    k_clock_finish<<<blocks(c->nscen, 256), 256, 0, s>>>(c->clk, c->nscen, phys(c));
+    k_clock_finish<<<blocks(c->nscen, 256), 256, 0, s>>>(c->clk, c->nscen, phys(c), barrier_timeout(c));
     c->launches++;
     CK(cudaGetLastError());
     CK(cudaEventRecord(c->ev1, s));

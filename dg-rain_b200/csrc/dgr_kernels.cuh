@@ -787,12 +787,13 @@ __global__ void __launch_bounds__(64, 8) k_fold_limit(const __grid_constant__ Me
 
 /* End of a step: step counter and the pending CFL update, taken by whichever clock kernel
  * comes next (the next step's, or k_clock_finish).  A scenario whose step just failed stops
- * here, so its step count is the number of steps that completed. */
-DGR_DEV void clock_end_item(DevClock *c)
+ * here, so its step count is the number of steps that completed; a step of the persistent
+ * kernels that left at a barrier's time-out (timed_out) did not complete and is not counted. */
+DGR_DEV void clock_end_item(DevClock *c, bool timed_out = false)
 {
     if (!c->in_step) return;
     c->in_step = 0;
-    if (c->done) return;
+    if (c->done || timed_out) return;
     if (c->err != ~0ull) {
         c->done = 1;
         return;
@@ -806,15 +807,17 @@ DGR_DEV void clock_end_item(DevClock *c)
  * scenario: take the end of the previous step, finish its CFL dt, stop when time has reached
  * final_time, evaluate the boundary values for this step (boundary_conditions() at the
  * current time), then advance the clock.  One block; thread s owns scenario s's clock,
- * then all threads write the prescribed edges.
+ * then all threads write the prescribed edges.  timeout: the barrier's time-out flag where
+ * the persistent kernels run, else null.
  */
 DGR_DEV void clock_begin_body(DevClock *clk, int nscen, const PhysParams &p, const int *__restrict__ bnd_edges,
                               const int *__restrict__ bnd_type, const int *__restrict__ bnd_sid, int nbnd,
-                              double *__restrict__ bzeta, double *__restrict__ bqn)
+                              double *__restrict__ bzeta, double *__restrict__ bqn, const unsigned *timeout)
 {
+    const bool timed_out = timeout && *(const volatile unsigned *)timeout;
     for (int s = threadIdx.x; s < nscen; s += blockDim.x) {
         DevClock *c = clk + s;
-        clock_end_item(c);
+        clock_end_item(c, timed_out);
         if (c->done) continue;
         if (c->dt_pending) {
             const double lam = __longlong_as_double((long long)c->lam_bits[p.stages - 1]);
@@ -853,20 +856,20 @@ static __global__ void __launch_bounds__(256) k_clock_begin(DevClock *clk, int n
                                                      const int *bnd_edges,
                                                      const int *bnd_type,
                                                      const int *bnd_sid, int nbnd,
-                                                     double *bzeta, double *bqn)
+                                                     double *bzeta, double *bqn, const unsigned *timeout)
 {
     pdl_wait();
     pdl_trigger();
-    clock_begin_body(clk, nscen, p, bnd_edges, bnd_type, bnd_sid, nbnd, bzeta, bqn);
+    clock_begin_body(clk, nscen, p, bnd_edges, bnd_type, bnd_sid, nbnd, bzeta, bqn, timeout);
 }
 
 /* After a run: derive each scenario's next dt so the host sees it. */
-static __global__ void k_clock_finish(DevClock *clk, int nscen, PhysParams p)
+static __global__ void k_clock_finish(DevClock *clk, int nscen, PhysParams p, const unsigned *timeout)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= nscen) return;
     DevClock *c = clk + s;
-    clock_end_item(c);
+    clock_end_item(c, timeout && *timeout);
     if (c->dt_pending) {
         const double lam = __longlong_as_double((long long)c->lam_bits[p.stages - 1]);
         double dt = p.cfl * c->min_edge / lam;
@@ -995,7 +998,8 @@ __global__ void __launch_bounds__(BS, 512 / BS) k_step_fused(const __grid_consta
 {
     if (with_clock) {
         if (blockIdx.x == 0)
-            clock_begin_body(a.clk, a.nscen, a.p, a.bnd_edges, a.bnd_type, a.bnd_sid, a.nbnd, a.bzeta, a.bqn);
+            clock_begin_body(a.clk, a.nscen, a.p, a.bnd_edges, a.bnd_type, a.bnd_sid, a.nbnd, a.bzeta, a.bqn,
+                             a.bar + 2);
         if (!grid_barrier(a.bar, a.bar_polls, a.bar_phantom)) return;
     }
     const int stride = gridDim.x * BS;

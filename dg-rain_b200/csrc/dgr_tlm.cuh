@@ -156,7 +156,7 @@ static __global__ void __launch_bounds__(256) k_adj_clock_begin(DevClock *clk, i
         time_hist[row + s] = clk[s].time;
     }
     __syncthreads();
-    clock_begin_body(clk, nscen, p, bnd_edges, bnd_type, bnd_sid, nbnd, bzeta, bqn);
+    clock_begin_body(clk, nscen, p, bnd_edges, bnd_type, bnd_sid, nbnd, bzeta, bqn, nullptr);
     /* thread s advanced scenario s's clock in clock_begin_body */
     if (!replay)
         for (int s = threadIdx.x; s < nscen; s += blockDim.x) dt_hist[row + s] = clk[s].dt;
