@@ -108,6 +108,16 @@ bool is_fresh(const void *p, size_t bytes)
     return absent > 4;
 }
 
+/* whether two copies have host bytes in common: copies down must then land in their order */
+bool overlap(const HostCopy *p, int n)
+{
+    for (int i = 0; i < n; ++i)
+        for (int j = 0; j < i; ++j)
+            if ((char *)p[i].host < (char *)p[j].host + p[j].bytes && (char *)p[j].host < (char *)p[i].host + p[i].bytes)
+                return true;
+    return false;
+}
+
 }  // namespace
 
 void stager_release(dgr_ctx *c)
@@ -150,9 +160,10 @@ cudaError_t host_copies(dgr_ctx *c, const HostCopy *p, int n, bool down)
     HostCopy threaded[kMaxHostCopies];
     int k = 0;
     size_t bytes = 0;
+    const bool apart = st && !(down && overlap(p, n));
     for (int i = 0; i < n; ++i) {
         if (!p[i].bytes) continue;
-        if (st && p[i].bytes >= kFreshBytes / 8 && !is_pinned(p[i].host)) {
+        if (apart && p[i].bytes >= kFreshBytes / 8 && !is_pinned(p[i].host)) {
             threaded[k++] = p[i];
             bytes += p[i].bytes;
         }
