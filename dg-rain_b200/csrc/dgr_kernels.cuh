@@ -664,8 +664,8 @@ struct NodeFold {
         for (int k = 0; k < 3; ++k) {
             b[k] = m.n2e_ptr[nd[k]];
             e[k] = m.n2e_ptr[nd[k] + 1];
-            if (!(index_ok(m, b[k], 3 * m.ne + 1, KID_NODE, el) && index_ok(m, e[k], 3 * m.ne + 1, KID_NODE, el) &&
-                  index_ok(m, e[k] - b[k], 3 * m.ne + 1, KID_NODE, el)))
+            if (!(index_ok(m, b[k], 3 * m.ne + 1, KID_LIMIT, el) && index_ok(m, e[k], 3 * m.ne + 1, KID_LIMIT, el) &&
+                  index_ok(m, e[k] - b[k] - 1, 3 * m.ne, KID_LIMIT, el))) /* the element itself is in the list */
                 return false;
         }
 #pragma unroll
@@ -673,7 +673,7 @@ struct NodeFold {
 #pragma unroll
             for (int j = 0; j < kFirst; ++j) {
                 id[k][j] = m.n2e[b[k] + j < e[k] ? b[k] + j : b[k]];
-                if (!index_ok(m, id[k][j], m.ne, KID_NODE, el)) return false;
+                if (!index_ok(m, id[k][j], m.ne, KID_LIMIT, el)) return false;
             }
         return true;
     }
@@ -686,7 +686,7 @@ struct NodeFold {
             if (a > mx[v][k]) mx[v][k] = a;
         }
     }
-    DGR_DEV void take(const MeshDev &m, const double *avg, int el)
+    DGR_DEV bool take(const MeshDev &m, const double *avg, int el)
     {
 #pragma unroll
         for (int v = 0; v < 3; ++v)
@@ -703,8 +703,10 @@ struct NodeFold {
         for (int k = 0; k < 3; ++k)
             for (int j = b[k] + kFirst; j < e[k]; ++j) {
                 const int next = m.n2e[j];
-                if (index_ok(m, next, m.ne, KID_NODE, el)) add(m, avg, k, next);
+                if (!index_ok(m, next, m.ne, KID_LIMIT, el)) return false;
+                add(m, avg, k, next);
             }
+        return true;
     }
 };
 
@@ -731,7 +733,7 @@ DGR_DEV void limit_item(const MeshDev &m, double *S, const double *bounds, const
     }
     if (ldm<COH>(&ck->done)) return;
     if (!nodes_ok || !fold_ok) return;
-    if (FOLD) fold.take(m, bounds, el);
+    if (FOLD && !fold.take(m, bounds, el)) return;
     const double zn[3] = {m.zn[nd[0]], m.zn[nd[1]], m.zn[nd[2]]};
     double w[3][3];
 #pragma unroll
