@@ -168,6 +168,15 @@ DGR_DEV void prefetch_geometry(const MeshDev &m, int base, int n)
 
 /* ------------------------------------------------------------------ edges ---- */
 
+/* whether an element's three edges are in range */
+DGR_DEV bool element_edges_ok(const MeshDev &m, int el)
+{
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        if (!index_ok(m, m.elem_edge[k * m.ldE + el] >> 1, m.nf, KID_ELEMENT, el)) return false;
+    return true;
+}
+
 /* One edge (2DCode/compute2DL.c:17-331): traces, ghost state, Roe flux(es); stores Fhat.n
  * for both sides and returns the edge's max wave speed (0 for a finished scenario).
  * FT: the numerical flux as a compile-time constant (0 Roe, 1 LLF, 2 HLLC), or -1 to take
@@ -567,7 +576,7 @@ __global__ void __launch_bounds__(96, 5)
         lam = fmax(fmax(fastest[0], fastest[1]), fastest[2]);
         if (lam > 0.0) atomicMax(&ck->lam_bits[lam_slot], (unsigned long long)__double_as_longlong(lam));
     }
-    if (k == 0 && live) {
+    if (k == 0 && live && element_edges_ok(m, el)) { /* a bad edge's flux was not taken */
         double F[3][3];
 #pragma unroll
         for (int v = 0; v < 3; ++v)

@@ -85,3 +85,21 @@ extern "C" unsigned long long dgr_t_bad_index(int where, int *touched)
     *touched = S != was || out[el] != -7;
     return bad;
 }
+
+/* the three edges of element 1 of 4, edge `at` (or none, -1) one past the last of 9 */
+extern "C" unsigned long long dgr_t_bad_edge(int at, int *ok)
+{
+    const int ne = 4, nf = 9, el = 1;
+    std::vector<int> ee(3 * ne);
+    for (int j = 0; j < 3 * ne; ++j) ee[j] = 2 * (j % nf) + j % 2;
+    if (at >= 0) ee[at * ne + el] = 2 * nf + 1;
+    unsigned long long bad = ~0ull;
+    MeshDev m;
+    memset(&m, 0, sizeof m);
+    m.ne = m.ldE = ne;
+    m.nf = nf;
+    m.elem_edge = ee.data();
+    m.bad_index = &bad;
+    *ok = element_edges_ok(m, el);
+    return bad;
+}

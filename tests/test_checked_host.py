@@ -1,6 +1,7 @@
 """The checked build's limiter that takes the node bounds itself, on the CPU: an index out of range
 among those it gathers is recorded under the limiter's kernel number and the element, and the
-element is left as it was."""
+element is left as it was; the element kernels' test of an element's three edges, at which an
+element whose flux was not taken is left alone."""
 from __future__ import annotations
 
 import ctypes as C
@@ -10,7 +11,7 @@ import subprocess
 import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-LIMITER, ELEMENT = 4, 1  # the kernel's number; the element that the harness runs
+LIMITER, ELEMENTS, ELEMENT = 4, 2, 1  # the kernels' numbers; the element that the harness runs
 
 
 @pytest.fixture(scope="module")
@@ -21,7 +22,7 @@ def lib(tmp_path_factory):
                     "-D__forceinline__=inline", "-D__shared__=static", "-D__launch_bounds__(...)=", "-o", path,
                     os.path.join(HERE, "checked_host.cpp")], check=True)
     lib = C.CDLL(path)
-    lib.dgr_t_bad_index.restype = C.c_ulonglong
+    lib.dgr_t_bad_index.restype = lib.dgr_t_bad_edge.restype = C.c_ulonglong
     return lib
 
 
@@ -36,3 +37,11 @@ def test_bad_index_is_the_limiters(lib, where):
     touched = C.c_int()
     assert lib.dgr_t_bad_index(where, C.byref(touched)) == LIMITER << 32 | ELEMENT
     assert not touched.value
+
+
+@pytest.mark.parametrize("at", [-1, 0, 1, 2])
+def test_bad_edge_of_an_element(lib, at):
+    ok = C.c_int()
+    want = 2**64 - 1 if at < 0 else ELEMENTS << 32 | ELEMENT
+    assert lib.dgr_t_bad_edge(at, C.byref(ok)) == want
+    assert ok.value == (at < 0)
