@@ -958,6 +958,15 @@ static int kernels_of_stages(const dgr_ctx *c)
     return n;
 }
 
+/* whether a launch of the separate kernels follows the schedule's block size */
+static bool block_size_matters(const dgr_ctx *c)
+{
+    if (c->p.order == 2) return false;
+    bool matters = !limiter_folds_nodes(c);
+    for (int st = 0; st < c->p.rk_stages; ++st) matters |= !edges_with_elements(c, stage_io(c, st));
+    return matters;
+}
+
 /* one RK stage as two to four kernels (buffers of stage_io) */
 void launch_stage(dgr_ctx *c, int stage, bool count)
 {
@@ -1543,6 +1552,10 @@ static int autotune_trials(dgr_ctx *c, int trial_steps, double *saveU, int *save
     std::vector<double> t(c->nscen), d(c->nscen), fin(c->nscen, 1e300);
     for (int b = 0; b < 3; ++b)
         for (int f = 0; f < (c->p.order == 2 ? 1 : 3); ++f) {
+            if (f == 0 && b > 0 && !block_size_matters(c)) { /* the launches of b = 0 */
+                if (ms_out) ms_out[3 * b] = ms_out[0];
+                continue;
+            }
             c->bs = bss[b];
             c->fusion = f;
             set_carveouts(c);
@@ -1551,7 +1564,7 @@ static int autotune_trials(dgr_ctx *c, int trial_steps, double *saveU, int *save
                 t[k] = clk0[k].time;
                 d[k] = clk0[k].dt > 0 ? clk0[k].dt : c->p.dt0;
             }
-            /* one untimed step builds the graph and warms the caches */
+            /* one untimed step warms the caches */
             int rc = run_impl(c, 1, fin.data(), t.data(), d.data(), nullptr);
             double ms = -1.0;
             if (rc == DGR_OK) {
