@@ -19,10 +19,13 @@
  *
  * Schedules of the device loop ("fusion depth"), chosen by dgr_autotune or
  * dgr_set_schedule:
- *   0: nine kernels per step at two stages (clock, 4 per stage), one thread per item;
+ *   0: separate kernels, one thread per item: the clock and four per stage (nine per step at
+ *      two stages), three per stage up to DGR_FOLD_LIMIT_MAX elements and two up to
+ *      DGR_EDGE_ELEMENT_MAX with the Roe flux, p = 2 always two;
  *   1: one persistent cooperative kernel per RK stage after the clock kernel;
  *   2: one persistent cooperative kernel per step, clock included;
- * and the block size (elements per block) of the element and limiter work.
+ * and the block size (elements per block) of the element and limiter work: of the persistent
+ * kernels, and of the separate element and limiter kernels where a step has them.
  */
 #include <cuda_runtime.h>
 
@@ -220,7 +223,10 @@ static int upload_concat(cudaStream_t s, T *dst, int nscen, const T *const *src,
  * twice.  us per step with a launch of each kind, with the limiter's fold, with both: 1,600
  * triangles 44.6, 42.7, 36.8; 8,000 48.7, 46.0, 45.0; 16,000 52.5, 49.6, 50.3; 24k 57.3, 53.7,
  * 62.7; 50,000 68.5, 64.9, 77.4; RK3 HLLC 6,000 51.1, 44.5, 45.5 and 91k 113.4, 110.1, 124.7;
- * 200k 165.7, 170.0, 246. */
+ * 200k 165.7, 170.0, 246.  The limiter's fold between its line and 200k: 110,000 116.5 without,
+ * 114.0 with; 130,000 131.9 and 131.5; 150,000 136.8 and 138.0; 175,000 152.4 and 157.9; RK3 HLLC
+ * 110,000 132.7 and 127.9, 150,000 151.9 and 151.0: even at 130,000 to 150,000; below, the line
+ * leaves 2-4 % unused. */
 #ifndef DGR_EDGE_ELEMENT_MAX
 #define DGR_EDGE_ELEMENT_MAX 8000
 #endif
@@ -1525,7 +1531,8 @@ extern "C" int dgr_get_schedule(const dgr_ctx *c, int *block_size, int *fusion)
 
 /*
  * Autotuner: times trial_steps steps of the device loop for every schedule (block size
- * 64/128/256 x fusion depth 0/1/2) from the current state, restoring state, flags and
+ * 64/128/256 x fusion depth 0/1/2; at fusion 0 once where the block size changes no launch)
+ * from the current state, restoring state, flags and
  * clocks after each trial, and keeps the fastest.  Results do not depend on the schedule
  * (same items, same arithmetic); only the time does.  ms_out (9 entries, or NULL)
  * receives the ms per step of each trial at index 3*b + f (b: 64, 128, 256; f: fusion),
@@ -1654,9 +1661,9 @@ extern "C" void dgr_host_free(void *p)
 
 /*
  * Per-kernel device timing of whole steps: CUDA events around every launch of nsteps
- * steps (dt of the last run, or dt0) with the four-kernel schedule.  kernel_ms[0..3]
- * receive the average ms of one launch of: edge flux, element RHS+RK, node bounds,
- * limiter+PDop.
+ * steps (dt of the last run, or dt0) with the four-kernel schedule, also on the small meshes
+ * whose own steps join some of these kernels.  kernel_ms[0..3] receive the average ms of one
+ * launch of: edge flux, element RHS+RK, node bounds, limiter+PDop.
  */
 /* dgr_profile_step of the p = 2 step: kernel_ms[0] edge fluxes, [1] element update */
 static int profile_p2(dgr_ctx *c, int nsteps, double *kernel_ms)

@@ -235,7 +235,7 @@ int upload_scenarios(dgr_ctx *c, int s0, int s1, const double *zeta, const doubl
                      const int *WD);             /* state of scenarios [s0, s1), reference layout */
 int read_clock(dgr_ctx *c);                      /* device clocks -> h_clk (synchronises) */
 int write_clock(dgr_ctx *c);                     /* h_clk -> device clocks (synchronises) */
-void launch_stage(dgr_ctx *c, int stage, bool count); /* one RK stage, four kernels */
+void launch_stage(dgr_ctx *c, int stage, bool count); /* one RK stage, two to four kernels */
 void launch_edge(dgr_ctx *c, const double *S, const int *wd, int lam_slot, int phase); /* p = 1 edge fluxes */
 bool edges_with_elements(const dgr_ctx *c);       /* p = 1: edges and elements share a launch */
 void launch_edge_element(dgr_ctx *c, int mode, const double *S, const double *U, const int *wd, double *OUT, double *avg,

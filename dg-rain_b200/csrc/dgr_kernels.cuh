@@ -310,8 +310,8 @@ DGR_DEV void copy_async4(int *dst, const int *src)
  * tiles, with the next tile's traces, geometry and flags on their way to shared memory
  * (cp.async, every thread its own edge's: no barrier) and the indices of the one after in
  * registers while a tile is computed.  The kernel is bound by FP64 dependency chains and was
- * waiting for the gathers behind the indices as much (4.3 cycles per issue); with them in
- * flight 16 warps per SM at 128 registers, without most spills, beat 24 at 80.  Against one
+ * waiting for the gathers behind the indices as much (4.2 stalled warps per issue at 1M triangles,
+ * 2.2 with them in flight); 16 warps per SM at 128 registers, without most spills, beat 24 at 80.  Against one
  * edge per thread, per step: 4M triangles 2.197 -> 2.137 ms, 200k 171 -> 166 us, RK3 HLLC 91k
  * 114 -> 111, ensemble of 32 (0.9M) 482 -> 469, 24k 58.1 -> 57.9, 1,600 45.1 -> 45.0. */
 template <bool WD, int FT, bool ENS>

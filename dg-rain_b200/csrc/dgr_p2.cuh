@@ -35,8 +35,9 @@ namespace dgr {
 /* Minimum resident blocks per SM requested for the p = 2 kernels (register caps 65536 /
  * (block size x blocks): 128 for the element kernel, 168 for the edge kernel at 128
  * threads), chosen by a measured sweep (163k triangles, SSP(3,3), us per step: edge kernel
- * 196.6 with three blocks, 199.0 with four, 227.9 with five; element kernel 225.4 with four,
- * 224.0 with three, 232.6 with five); overridable at build time. */
+ * 196.6 with three blocks, 199.0 with four, 227.9 with five; element kernel 196.4 with three,
+ * 197.4 with four, 207.7 with five: three and four are 0.5 % apart, and four's 40 B of spills
+ * against none do not show); overridable at build time. */
 #ifndef DGR_P2_MINB_EDGE
 #define DGR_P2_MINB_EDGE 3
 #endif

@@ -430,11 +430,10 @@ DGR_HD void element_core(const T F[3][3], const T zr[3], const T qxr[3], const T
 #pragma unroll
             for (int k = 0; k < 3; ++k) w[v][k] = a * uin(v, k) + b * (s[v][k] + rhs[v][k] * dt);
     }
-    if constexpr (RCP) { /* the means' divisions by 3 through the reciprocal RN(1/3) */
-        bool ok_avg = true;
+    if constexpr (RCP) { /* the means' divisions by 3 through the reciprocal RN(1/3), valid everywhere */
 #pragma unroll
         for (int v = 0; v < 3; ++v) avg[v] = third(w[v][0] + w[v][1] + w[v][2]);
-        *rcp_ok = ok && ok_avg;
+        *rcp_ok = ok;
     } else {
 #pragma unroll
         for (int v = 0; v < 3; ++v) avg[v] = (w[v][0] + w[v][1] + w[v][2]) / 3;

@@ -257,7 +257,8 @@ class Solver:
         return float(self.lib.dgr_last_device_ms(self.ctx))
 
     def profile_step(self, nsteps: int = 3):
-        """Average device ms per launch of (edge flux, element, node bounds, limiter)."""
+        """Average device ms per launch of (edge flux, element, node bounds, limiter), the separate
+        kernels at every mesh size (the steps of small meshes join some of them)."""
         out = (C.c_double * 4)()
         self._status(self.lib.dgr_profile_step(self.ctx, nsteps, out, 4), "dgr_profile_step")
         return list(out)
@@ -275,8 +276,9 @@ def _schedule_methods(cls):
         return b.value, f.value
 
     def autotune(self, trial_steps: int = 5):
-        """Times every schedule from the current state (restored afterwards) and keeps the
-        fastest; returns (block_size, fusion, {(block_size, fusion): ms per step})."""
+        """Times every schedule from the current state (restored afterwards; those whose launches
+        are the same once) and keeps the fastest; returns (block_size, fusion, {(block_size,
+        fusion): ms per step})."""
         b, f = C.c_int(), C.c_int()
         ms = (C.c_double * 9)()
         _lib.check(self.lib.dgr_autotune(self.ctx, trial_steps, C.byref(b), C.byref(f), ms), "dgr_autotune")

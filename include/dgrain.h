@@ -222,6 +222,9 @@ DGR_API void dgr_host_free(void *p);
 /* ---- device context ------------------------------------------------------------- */
 
 DGR_API int dgr_params_default(dgr_params *p);
+/* A context of 4 MB of state or more also takes 4 MB of page-locked host memory: through it up to
+ * four threads, started and ended within a call, share the copies of large pageable arrays (where
+ * the calling thread may use three CPUs or more; into pages not there yet, always). */
 DGR_API int dgr_create(const dgr_mesh_view *mesh, const dgr_params *params, dgr_ctx **out);
 DGR_API int dgr_destroy(dgr_ctx *ctx);
 DGR_API int dgr_get_params(const dgr_ctx *ctx, dgr_params *out);
@@ -244,7 +247,9 @@ DGR_API int dgr_set_boundary(dgr_ctx *ctx, const double *bzeta, const double *bQ
 /* ... or the device fills them for time t from the reference constants and the tide. */
 DGR_API int dgr_boundary_conditions(dgr_ctx *ctx, double time);
 
-/* Single operators on the device state, for drop-in use and parity checks. */
+/* Single operators on the device state, for drop-in use and parity checks.  dgr_compute_L keeps
+ * 72 B per element (144 at p = 2) of device memory from the first call that asks for its arrays
+ * until dgr_destroy. */
 DGR_API int dgr_compute_L(dgr_ctx *ctx, double time, double *RHSZeta, double *RHSQx, double *RHSQy,
                   double *max_lambda);
 DGR_API int dgr_slope_limiter(dgr_ctx *ctx);
@@ -261,7 +266,9 @@ DGR_API int dgr_step(dgr_ctx *ctx, double time, double dt, double *max_lambda);
 /* time_evolution(): up to nsteps steps while time < final_time, entirely on the device
  * (CFL dt, boundary forcing and clock stay on the GPU; one host sync at the end).
  * *time_io < 0 starts a new run at t = 0 with dt = dt0; otherwise (*time_io, *dt_io)
- * continue a previous run.  The steps of one call are replayed from a CUDA graph. */
+ * continue a previous run.  Calls of 16 steps or more replay a CUDA graph of eight; what does
+ * not fill one, and shorter calls, are launched step by step.  After DGR_ERR_TIMEOUT
+ * (dgr_set_barrier_wait) *steps_done leaves out the steps that timed out. */
 DGR_API int dgr_run(dgr_ctx *ctx, int nsteps, double final_time, double *time_io, double *dt_io,
             int *steps_done);
 
@@ -286,12 +293,15 @@ DGR_API int dgr_ensemble_run(dgr_ctx *ctx, int nsteps, const double *final_time,
 DGR_API int dgr_ensemble_last_error(dgr_ctx *ctx, int scenario, int *code, int *index, int *step);
 
 /* Schedule of the device loop: block size (elements per block of the element and limiter
- * work: 64, the default, 128 or 256) and fusion depth (0, the default: ten kernels per
- * step; 1: one persistent cooperative kernel per RK stage; 2: one per step, clock
- * included).  dgr_autotune times
+ * work: 64, the default, 128 or 256) and fusion depth (0, the default: separate kernels, nine
+ * per step at two stages, seven up to 100,000 elements, five up to 8,000 with the Roe flux;
+ * 1: one persistent cooperative kernel per RK stage; 2: one per step, clock included).  At
+ * fusion 0 the joined kernels of the smaller meshes, and those of p = 2, have block sizes of
+ * their own.  dgr_autotune times
  * trial_steps steps of every schedule from the current state (restored afterwards),
  * keeps the fastest and reports it; ms_out (9 entries or NULL) gets ms per step at index
- * 3*b + f, b = 0,1,2 for 64,128,256.  Results do not depend on the schedule. */
+ * 3*b + f, b = 0,1,2 for 64,128,256.  Schedules whose launches are the same are timed once and
+ * reported alike.  Results do not depend on the schedule. */
 DGR_API int dgr_set_schedule(dgr_ctx *ctx, int block_size, int fusion);
 DGR_API int dgr_get_schedule(const dgr_ctx *ctx, int *block_size, int *fusion);
 /* Bound of the persistent kernels' grid-barrier wait (fusion 1 and 2): a block that polls
@@ -323,7 +333,8 @@ DGR_API long long dgr_kernel_launches(const dgr_ctx *ctx);
 DGR_API double dgr_last_device_ms(const dgr_ctx *ctx);
 /* Runs nsteps steps with CUDA events around every launch; kernel_ms[0..3] (n >= 4)
  * receive the average ms of one launch of: edge flux, element RHS + RK update, node
- * bounds, limiter + PDop. */
+ * bounds, limiter + PDop (p = 2: edge flux, element update, 0, 0).  These are the separate
+ * kernels at every mesh size; up to 100,000 elements a step of dgr_run joins some of them. */
 DGR_API int dgr_profile_step(dgr_ctx *ctx, int nsteps, double *kernel_ms, int n);
 
 /* Slope limiter without any device allocation.  This entry point has no counterpart in
